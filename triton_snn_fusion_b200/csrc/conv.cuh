@@ -36,6 +36,10 @@ struct ConvArgs {
 // CUDA-core implicit GEMM (any shape, fp32 accumulate).
 int conv_lif_simt(const ConvArgs &a, cudaStream_t stream);
 
+// The fp32 form of it with asynchronous copies and packed multiply-adds; conv_lif_simt hands it the calls it takes.
+bool conv_f32_supported(const ConvArgs &a);
+int conv_f32(const ConvArgs &a, cudaStream_t stream);
+
 // Direct CUDA-core kernel for 3x3 convs over images with at most four channels (the first layer of a network).
 bool conv_smallcin_supported(const ConvArgs &a);
 int conv_smallcin(const ConvArgs &a, cudaStream_t stream);
