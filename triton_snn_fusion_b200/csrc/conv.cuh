@@ -58,8 +58,14 @@ int halo_device_status(int *out);
 // the pixels of two timesteps as a 256-wide N operand (the only shape that runs the tensor pipe at
 // its full rate), halo tiles in shared memory. Preferred over conv3x3_halo when supported.
 bool conv3x3_pair_supported(const ConvArgs &a);
+bool pair_shape_supported(const ConvArgs &a);   // all of it but the number of timesteps
 int conv3x3_pair(const ConvArgs &a, cudaStream_t stream);
 int pair_device_status(int *out);
+// The form of it for calls with few output tiles (conv_split.cu): the reduction of a tile over a cluster of CTAs.
+// conv_split_plan returns the cluster size, 0 where the timestep-pair kernel itself is the better one.
+int conv_split_plan(const ConvArgs &a);
+int conv_split(const ConvArgs &a, int S, cudaStream_t stream);
+int split_device_status(int *out);
 // Self-test of the bounded waits (snnb_selftest_arm_wait_timeout): if armed, hands the shortened limit and the
 // "drop one load" switch to the next launch of the timestep-pair kernel and disarms.
 void consume_wait_selftest(long long *limit_cycles, int *drop_load);

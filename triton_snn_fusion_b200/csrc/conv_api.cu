@@ -21,6 +21,8 @@ int run(const ConvArgs &a, int path, cudaStream_t stream, const char *what) {
   if (path == SNNB_PATH_AUTO && conv_smallcin_supported(a)) return conv_smallcin(a, stream);   // RGB first layers
   if (path == SNNB_PATH_SIMT) return conv_lif_simt(a, stream);
   const bool taps_only = path == SNNB_PATH_TCGEN05_TAPS;
+  if (!taps_only && path != SNNB_PATH_TCGEN05_HALO)
+    if (const int S = conv_split_plan(a)) return conv_split(a, S, stream);
   if (!taps_only && path != SNNB_PATH_TCGEN05_HALO && conv3x3_pair_supported(a)) return conv3x3_pair(a, stream);
   if (!taps_only && conv3x3_halo_supported(a)) return conv3x3_halo(a, stream);
   const char *why = "";
@@ -84,7 +86,7 @@ extern "C" int snnb_conv_lif_which(int T, int B, int Cin, int H, int W, int Cout
   const char *why = "";
   if (path == SNNB_PATH_AUTO && conv_smallcin_supported(a)) k = "conv3x3_smallcin";
   else if (path == SNNB_PATH_SIMT) k = "conv_lif_simt";
-  else if (!taps_only && path != SNNB_PATH_TCGEN05_HALO && conv3x3_pair_supported(a)) k = "conv3x3_pair";
+  else if (!taps_only && path != SNNB_PATH_TCGEN05_HALO && (conv3x3_pair_supported(a) || conv_split_plan(a))) k = "conv3x3_pair";
   else if (!taps_only && conv3x3_halo_supported(a)) k = "conv3x3_halo";
   else if (conv_lif_tc_supported(a, &why)) k = "conv_lif_tc";
   else if (path != SNNB_PATH_AUTO) return fail(SNNB_ERR_UNSUPPORTED, "conv_lif_which: no tensor-core kernel takes this call: %s", why);
@@ -124,6 +126,7 @@ extern "C" int snnb_conv3x3_shortcut_lif(const void *x_seq, int64_t x_t_stride, 
                 "conv and snnb_conv_lif with a residual instead");
   if (membranes_overlap_partially(a))
     return fail(SNNB_ERR_INVALID, "conv3x3_shortcut_lif: v_init and v_out overlap without being the same buffer");
+  if (const int S = conv_split_plan(a)) return conv_split(a, S, static_cast<cudaStream_t>(stream));
   return conv3x3_pair(a, static_cast<cudaStream_t>(stream));
 }
 
@@ -145,8 +148,8 @@ extern "C" int snnb_linear_lif(const void *x_seq, int64_t x_t_stride, const void
   a.x = x_seq; a.x_t_stride = x_t_stride; a.w = w; a.b = b; a.res = nullptr;
   a.v_init = v_init; a.spikes = spikes; a.v_out = v_out;
   // a 1x1 conv over the tokens laid out as an image: 8 tokens per row when that divides (the shape the
-  // timestep-pair kernel tiles), else one row of M tokens
-  const bool rows8 = M % 8 == 0 && M >= 64;
+  // timestep-pair kernel tiles; at most 56 tokens are one of its whole small maps), else one row of M tokens
+  const bool rows8 = M % 8 == 0;
   a.T = T; a.B = 1; a.Cin = K; a.H = rows8 ? M / 8 : 1; a.W = rows8 ? 8 : M; a.Cout = N; a.KH = 1; a.KW = 1;
   a.stride = 1; a.pad = 0; a.Ho = a.H; a.Wo = a.W; a.lif = 1;
   a.dtype = dtype; a.spike_dtype = spike_dtype; a.v_dtype = v_dtype;

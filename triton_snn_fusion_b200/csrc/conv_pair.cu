@@ -27,7 +27,7 @@ void consume_wait_selftest(long long *limit_cycles, int *drop_load) {
 SNNB_PAIR_UNITS(SNNB_PAIR_DECL)
 #undef SNNB_PAIR_DECL
 
-bool conv3x3_pair_supported(const ConvArgs &a) {
+bool pair_shape_supported(const ConvArgs &a) {
   if (a.dtype != SNNB_BF16 && a.dtype != SNNB_F16) return false;
   const bool k3 = a.KH == 3 && a.KW == 3 && a.stride == 1 && a.pad == 1;
   const bool k1 = a.KH == 1 && a.KW == 1 && a.stride == 1 && a.pad == 0;   // reads only the centre of each halo tile
@@ -41,9 +41,6 @@ bool conv3x3_pair_supported(const ConvArgs &a) {
   if (a.Cin % 8 != 0) return false;
   if (a.Cin % 64 != 0 && (a.KH != 1 || a.sc_x != nullptr)) return false;   // only the 1x1 form has been checked on partial slabs
   if (a.x_t_stride == 0 && a.T > 1) return false;   // one frame for all steps: left to the other kernels
-  // T = 1, or an even number of steps: they are processed as pairs that alternate between two accumulators in
-  // tensor memory while the membrane stays in registers, so any number of pairs fits
-  if (a.T != 1 && (a.T % 2 != 0 || a.T > 64)) return false;
   // maps of at least 8 x 8 (one image per tile) or at most 7 x 8 (two images per tile, Cout > 64); what lies
   // in between goes to conv_halo.cu
   const bool one_image = a.Ho >= 8 && a.Wo >= 8;
@@ -58,6 +55,12 @@ bool conv3x3_pair_supported(const ConvArgs &a) {
     if (a.sc_t_stride % 8 != 0 || a.sc_t_stride <= 0 || !aligned16(a.sc_x) || !aligned16(a.sc_w)) return false;
   }
   return true;
+}
+
+// T = 1, or an even number of steps: they are processed as pairs that alternate between two accumulators in
+// tensor memory while the membrane stays in registers, so any number of pairs fits
+bool conv3x3_pair_supported(const ConvArgs &a) {
+  return pair_shape_supported(a) && (a.T == 1 || (a.T % 2 == 0 && a.T <= 64));
 }
 
 int conv3x3_pair(const ConvArgs &a, cudaStream_t stream) {

@@ -436,7 +436,10 @@ extern "C" int snnb_device_status(int *status_out) {
   int h5 = 0;
   const int rc5 = dw_device_status(&h5);
   if (rc5 != SNNB_OK) return rc5;
-  *status_out = h | h2 | h3 | h4 | h5;
+  int h6 = 0;
+  const int rc6 = split_device_status(&h6);
+  if (rc6 != SNNB_OK) return rc6;
+  *status_out = h | h2 | h3 | h4 | h5 | h6;
   return SNNB_OK;
 }
 
