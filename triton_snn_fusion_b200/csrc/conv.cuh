@@ -61,6 +61,10 @@ bool conv3x3_pair_supported(const ConvArgs &a);
 bool pair_shape_supported(const ConvArgs &a);   // all of it but the number of timesteps
 int conv3x3_pair(const ConvArgs &a, cudaStream_t stream);
 int pair_device_status(int *out);
+// The form of it for 1x1 convs and linear layers, any T (conv_pw.cu).
+bool conv_pw_supported(const ConvArgs &a);
+int conv_pw(const ConvArgs &a, cudaStream_t stream);
+int pw_device_status(int *out);
 // The form of it for calls with few output tiles (conv_split.cu): the reduction of a tile over a cluster of CTAs.
 // conv_split_plan returns the cluster size, 0 where the timestep-pair kernel itself is the better one.
 int conv_split_plan(const ConvArgs &a);

@@ -21,8 +21,10 @@ int run(const ConvArgs &a, int path, cudaStream_t stream, const char *what) {
   if (path == SNNB_PATH_AUTO && conv_smallcin_supported(a)) return conv_smallcin(a, stream);   // RGB first layers
   if (path == SNNB_PATH_SIMT) return conv_lif_simt(a, stream);
   const bool taps_only = path == SNNB_PATH_TCGEN05_TAPS;
-  if (!taps_only && path != SNNB_PATH_TCGEN05_HALO)
+  if (!taps_only && path != SNNB_PATH_TCGEN05_HALO) {
     if (const int S = conv_split_plan(a)) return conv_split(a, S, stream);
+    if (conv_pw_supported(a)) return conv_pw(a, stream);
+  }
   if (!taps_only && path != SNNB_PATH_TCGEN05_HALO && conv3x3_pair_supported(a)) return conv3x3_pair(a, stream);
   if (!taps_only && conv3x3_halo_supported(a)) return conv3x3_halo(a, stream);
   const char *why = "";
@@ -86,7 +88,7 @@ extern "C" int snnb_conv_lif_which(int T, int B, int Cin, int H, int W, int Cout
   const char *why = "";
   if (path == SNNB_PATH_AUTO && conv_smallcin_supported(a)) k = "conv3x3_smallcin";
   else if (path == SNNB_PATH_SIMT) k = "conv_lif_simt";
-  else if (!taps_only && path != SNNB_PATH_TCGEN05_HALO && (conv3x3_pair_supported(a) || conv_split_plan(a))) k = "conv3x3_pair";
+  else if (!taps_only && path != SNNB_PATH_TCGEN05_HALO && (conv3x3_pair_supported(a) || conv_pw_supported(a) || conv_split_plan(a))) k = "conv3x3_pair";
   else if (!taps_only && conv3x3_halo_supported(a)) k = "conv3x3_halo";
   else if (conv_lif_tc_supported(a, &why)) k = "conv_lif_tc";
   else if (path != SNNB_PATH_AUTO) return fail(SNNB_ERR_UNSUPPORTED, "conv_lif_which: no tensor-core kernel takes this call: %s", why);

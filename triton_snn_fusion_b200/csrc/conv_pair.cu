@@ -30,7 +30,7 @@ SNNB_PAIR_UNITS(SNNB_PAIR_DECL)
 bool pair_shape_supported(const ConvArgs &a) {
   if (a.dtype != SNNB_BF16 && a.dtype != SNNB_F16) return false;
   const bool k3 = a.KH == 3 && a.KW == 3 && a.stride == 1 && a.pad == 1;
-  const bool k1 = a.KH == 1 && a.KW == 1 && a.stride == 1 && a.pad == 0;   // reads only the centre of each halo tile
+  const bool k1 = a.KH == 1 && a.KW == 1 && a.stride == 1 && a.pad == 0;   // (conv_split.cu only)
   // stride 2: four phase views of the input per slab; the base of the odd-column views must stay 16-byte aligned
   const bool k3s2 = a.KH == 3 && a.KW == 3 && a.stride == 2 && a.pad == 1 && a.Cout > 64 && a.H >= 2 && a.W >= 2;
   if (!k3 && !k1 && !k3s2) return false;
@@ -60,7 +60,7 @@ bool pair_shape_supported(const ConvArgs &a) {
 // T = 1, or an even number of steps: they are processed as pairs that alternate between two accumulators in
 // tensor memory while the membrane stays in registers, so any number of pairs fits
 bool conv3x3_pair_supported(const ConvArgs &a) {
-  return pair_shape_supported(a) && (a.T == 1 || (a.T % 2 == 0 && a.T <= 64));
+  return a.KH == 3 && pair_shape_supported(a) && (a.T == 1 || (a.T % 2 == 0 && a.T <= 64));
 }
 
 int conv3x3_pair(const ConvArgs &a, cudaStream_t stream) {

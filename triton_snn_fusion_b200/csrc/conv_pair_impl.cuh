@@ -1,4 +1,4 @@
-// 3x3 / stride 1 / padding 1 conv (+ bias, + residual) + LIF over T steps (T = 1 or even) with the operand roles
+// 3x3 / padding 1 conv, stride 1 or 2 (+ bias, + residual) + LIF over T steps (T = 1 or even) with the operand roles
 // swapped so that one tcgen05.mma covers 256 output pixels.
 //
 // Measured on B200: a tcgen05.mma (cta_group::1, K = 16) occupies the tensor pipe for ~128 cycles
@@ -43,7 +43,6 @@ constexpr int kRowBytes = kPW * 128;                   // 1280
 constexpr int kHaloT = kPW * kPH * 128;                // 20480 bytes per timestep
 constexpr int kTileRows = 14;                          // valid output rows per tile
 constexpr int kPairRing = 3;                           // halo (pair) slots
-constexpr int kPairRingMax = 4;                        // ... four of the smaller halo-free tiles of 1x1 convs, which each feed one MMA group only
 constexpr int kIdentBytes = 192 * 128;                 // zero rows / 64x64 identity / zero rows, see the residual path
 constexpr int kWRingP = 5;                             // weight-tile slots (16 KB each): a load must cover ~1 us of L2 latency
 constexpr int kWBarsP = 8;                             // barrier pairs reserved for weight slots (the resident form uses six)
@@ -69,15 +68,8 @@ struct PairGeom {
   int s2;         // 3x3 / stride 2 / padding 1: per slab four halo tiles, one per phase (row parity a, column
                   // parity b) of the input, each seen through a tensor map with doubled strides; input row
                   // 2i - 1 + kh is phase row i - 1 (kh = 0, a = 1), i (kh = 1, a = 0) or i (kh = 2, a = 1)
-  int ntaps;      // 9 (3x3 conv) or 1 (1x1 conv / linear: only the centre of the halo tile is used)
   int sc_slabs;   // > 0: instead of a residual tensor, a 1x1 shortcut conv over sc_slabs 64-channel slabs of a
                   // second input is accumulated (its pixel tiles come through rmap, its weights through scwmap)
-  int flat;       // 1x1 conv on a map of at least 16 rows: the pixel tile is loaded without a halo (8 x 16 pixels, all
-                  // of them outputs) instead of as the centre of a 10 x 16 halo tile
-  int pw;         // pixels per tile row in shared memory: 10 (with halo) or 8 (flat)
-  int row_bytes;  // pw * 128
-  int halo_t;     // bytes of one timestep's tile: pw * 16 * 128
-  int tile_rows;  // output rows a tile produces: 14 (with halo) or 16 (flat)
   int ring;   // halo slots in use
   int wring;  // weight slots in use (<= kWBarsP)
   int wres;   // twin form without residual, one channel slab: the six weight tiles (96 KB) are loaded once per block and
@@ -107,7 +99,7 @@ struct PairGeom {
 // whose input rows / columns have the parity of phase ph = 2a + b.
 template <bool S2, bool TWIN>
 __device__ __forceinline__ int phase_ntaps(const PairGeom &g, int ph) {
-  return S2 ? ((ph & 2) ? 2 : 1) * ((ph & 1) ? 2 : 1) : (TWIN ? 6 : g.ntaps);
+  return S2 ? ((ph & 2) ? 2 : 1) * ((ph & 1) ? 2 : 1) : (TWIN ? 6 : 9);
 }
 // j-th tap of phase ph: its index in the weight tensor (kh * 3 + kw) and its row offset inside the halo tile.
 template <bool S2, bool TWIN>
@@ -122,9 +114,9 @@ __device__ __forceinline__ void phase_tap(const PairGeom &g, int ph, int j, int 
       off = (j < 3 ? 0 : kPW) + wtap;
       return;
     }
-    const int kh = g.ntaps == 1 ? 1 : j / 3, kw = g.ntaps == 1 ? 1 : j - kh * 3;
-    wtap = g.ntaps == 1 ? 0 : j;
-    off = g.flat ? 0 : kh * kPW + kw;
+    const int kh = j / 3, kw = j - kh * 3;
+    wtap = j;
+    off = kh * kPW + kw;
   } else {
     const int a = ph >> 1, b = ph & 1, nc = b ? 2 : 1;
     const int jr = j / nc, jc = j - jr * nc;
@@ -387,8 +379,12 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
                     ST *__restrict__ spikes, VT *v_out, const PairGeom g, const LifParams p) {
   using R = Roles<TWIN>;
   const bool dup = DUP || (S2 && g.dup);
+  // The nine-tap loops of the weight producer and the MMA issuer stay loops: unrolled they compete with the epilogue for
+  // the instruction cache (64 -> 128, 16x16, batch 415: 106 us as a loop, 123 us unrolled; the six groups of the twin form:
+  // 123 us as a loop, 117 us unrolled).
+  constexpr int kTapUnroll = TWIN ? 6 : (S2 ? 4 : 1);
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bars[2 * kPairRingMax + 2 * kWBarsP + 4];
+  __shared__ __align__(8) uint64_t bars[2 * kPairRing + 2 * kWBarsP + 4];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
 
@@ -400,14 +396,14 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
   const uint32_t ident_base = smem_base;
   const uint32_t w_base = smem_base + ((g.has_res && !g.sc_slabs) ? (uint32_t)(TWIN ? kTwinIdentBytes : kIdentBytes) : 0u);
   const uint32_t h_base = w_base + (uint32_t)(g.wring * kWSlot);
-  const uint32_t slot_bytes = (uint32_t)(g.tq * g.halo_t);
+  const uint32_t slot_bytes = (uint32_t)(g.tq * kHaloT);
   const uint32_t bar_base = umma::smem_u32(bars);
   auto hfull = [&](uint32_t s) { return bar_base + 8u * s; };
-  auto hempty = [&](uint32_t s) { return bar_base + 8u * ((uint32_t)kPairRingMax + s); };
-  auto wfull = [&](uint32_t s) { return bar_base + 8u * (2u * kPairRingMax + s); };
-  auto wempty = [&](uint32_t s) { return bar_base + 8u * (2u * kPairRingMax + kWBarsP + s); };
-  auto accfull = [&](uint32_t s) { return bar_base + 8u * (2u * kPairRingMax + 2u * kWBarsP + s); };
-  auto accempty = [&](uint32_t s) { return bar_base + 8u * (2u * kPairRingMax + 2u * kWBarsP + 2u + s); };
+  auto hempty = [&](uint32_t s) { return bar_base + 8u * ((uint32_t)kPairRing + s); };
+  auto wfull = [&](uint32_t s) { return bar_base + 8u * (2u * kPairRing + s); };
+  auto wempty = [&](uint32_t s) { return bar_base + 8u * (2u * kPairRing + kWBarsP + s); };
+  auto accfull = [&](uint32_t s) { return bar_base + 8u * (2u * kPairRing + 2u * kWBarsP + s); };
+  auto accempty = [&](uint32_t s) { return bar_base + 8u * (2u * kPairRing + 2u * kWBarsP + 2u + s); };
   volatile int *abort_flag = &abort_s;
   const long long wl = g.wait_limit;   // SM cycles after which a wait on an mbarrier gives up
 
@@ -429,9 +425,9 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
     // The last strip / row tile is shifted back inside the image instead of sticking out of it: it then
     // recomputes a few pixels of its neighbour (both write the same values) and every tile is complete.
     w0 = min(strip * 8, max(g.Wo - 8, 0));
-    h0 = min(rt * g.tile_rows, max(g.Ho - g.tile_rows, 0));
+    h0 = min(rt * kTileRows, max(g.Ho - kTileRows, 0));
     wlo = strip * 8;
-    hlo = rt * g.tile_rows;
+    hlo = rt * kTileRows;
   };
 
   if (threadIdx.x == 0) {
@@ -485,7 +481,6 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
     };
     uint32_t slot = 0, phase = 1;
     bool ok = true;
-    const int org = g.flat ? 0 : 1;   // the halo tile starts one pixel up and to the left of the output tile
     constexpr int nph = S2 ? 4 : 1;
     for (int tile = blockIdx.x; tile < g.total_tiles && ok; tile += gridDim.x) {
       int n0, w0, h0, b, wlo_unused, hlo_unused;
@@ -501,8 +496,8 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
           ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
           if (!ok) break;
           if (lane < g.tq) {
-            const uint32_t dst = h_base + slot * slot_bytes + (uint32_t)lane * (uint32_t)g.halo_t;
-            umma::tma_load_5d(dst, xm, hfull(slot), slab * 64, w0 - org, h0 - org, b, pair * g.tq + lane);
+            const uint32_t dst = h_base + slot * slot_bytes + (uint32_t)lane * (uint32_t)kHaloT;
+            umma::tma_load_5d(dst, xm, hfull(slot), slab * 64, w0 - 1, h0 - 1, b, pair * g.tq + lane);
             if (g.stack && b + 1 < g.B)
               umma::tma_load_5d(dst + 8u * kRowBytes, xm, hfull(slot), slab * 64, -1, -1, b + 1, pair * g.tq + lane);
           }
@@ -521,8 +516,8 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
           ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
           if (!ok) break;
           if (lane < g.tq) {
-            const uint32_t dst = h_base + slot * slot_bytes + (uint32_t)lane * (uint32_t)g.halo_t;
-            umma::tma_load_5d(dst, &rmap, hfull(slot), res_c0, w0 - org, h0 - org, b, pair * g.tq + lane);
+            const uint32_t dst = h_base + slot * slot_bytes + (uint32_t)lane * (uint32_t)kHaloT;
+            umma::tma_load_5d(dst, &rmap, hfull(slot), res_c0, w0 - 1, h0 - 1, b, pair * g.tq + lane);
             if (g.stack && b + 1 < g.B)
               umma::tma_load_5d(dst + 8u * kRowBytes, &rmap, hfull(slot), res_c0, -1, -1, b + 1, pair * g.tq + lane);
           }
@@ -541,6 +536,7 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
           if (TWIN && g.wres && (tile != (int)blockIdx.x || pair != 0)) continue;   // resident weights: loaded once
           for (int sp = 0; sp < g.kslabs * (S2 ? 4 : 1) && ok; ++sp) {
             const int slab = S2 ? sp >> 2 : sp, ph = S2 ? sp & 3 : 0;
+#pragma unroll kTapUnroll
             for (int j = 0; j < phase_ntaps<S2, TWIN>(g, ph); ++j) {
               int tap, off_unused;
               phase_tap<S2, TWIN>(g, ph, j, tap, off_unused);
@@ -586,7 +582,7 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
     if (lane == 0) {
       const uint32_t idesc = umma::make_idesc_f16(128, 128 * g.tq, std::is_same<XT, __nv_bfloat16>::value);
       uint64_t hdesc0 = umma::make_sw128_kmajor_desc(h_base);
-      hdesc0 = (hdesc0 & ~((uint64_t)0x3FFF << 32)) | ((uint64_t)(g.row_bytes >> 4) << 32);
+      hdesc0 = (hdesc0 & ~((uint64_t)0x3FFF << 32)) | ((uint64_t)(kRowBytes >> 4) << 32);
       const uint64_t wdesc0 = umma::make_sw128_kmajor_desc(w_base);
       uint32_t slot = 0, phase = 0, ws = 0, wphase = 0, it = 0;
       bool ok = true;
@@ -605,6 +601,7 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
             const int ph = S2 ? sp & 3 : 0;
             ok = umma::mbar_wait(hfull(slot), phase, abort_flag, wl);
             if (!ok) break;
+#pragma unroll kTapUnroll
             for (int tap = 0; tap < phase_ntaps<S2, TWIN>(g, ph); ++tap) {
               // resident weights: slot = tap, complete after the first pass over the six slots
               if (!(TWIN && g.wres) || (it == 0 && pair == 0)) ok = umma::mbar_wait(wfull(ws), wphase, abort_flag, wl);
@@ -641,7 +638,7 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
               adesc = umma::make_sw128_kmajor_desc(ident_base + ((rs == 0 && !dup && !TWIN) ? 64u * 128u : 0u));
             }
             umma::tc_fence_after_sync();
-            const uint64_t xdesc = hdesc0 + (uint64_t)((slot * slot_bytes + (g.flat ? 0u : (uint32_t)(kPW + 1) * 128u)) >> 4);
+            const uint64_t xdesc = hdesc0 + (uint64_t)((slot * slot_bytes + (uint32_t)(kPW + 1) * 128u) >> 4);
 #pragma unroll
             for (int k = 0; k < 4; ++k) umma::mma_f16_ss(d, adesc + (uint64_t)(2 * k), xdesc + (uint64_t)(2 * k), idesc, 1u);
             if (g.sc_slabs) {
@@ -785,7 +782,7 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
       const int c = n0 + ch_in_tile;                   // output channel of this thread
       const int img = g.stack ? b + (r_begin >> 3) : b;   // two images per tile: row groups 8.. belong to image b + 1
       const int row_first = g.stack ? 0 : h0 + r_begin;   // image row of this thread's first row group
-      const int row_limit = g.stack ? 8 : g.tile_rows - r_begin;   // row groups of this thread that can hold outputs
+      const int row_limit = g.stack ? 8 : kTileRows - r_begin;   // row groups of this thread that can hold outputs
       const bool c_ok = c < g.Cout && img < g.B;
       // the two biases of a conv with a fused shortcut conv are widened first and added in fp32
       const float bias_c = ((bias != nullptr && c_ok) ? DT<XT>::to_f(bias[c]) : 0.f) +
@@ -894,18 +891,12 @@ int launch(const ConvArgs &a, cudaStream_t stream) {
   g.Tacc = (a.x_t_stride == 0) ? 1 : a.T;
   g.B = a.B; g.Cin = a.Cin; g.Cout = a.Cout; g.Ho = a.Ho; g.Wo = a.Wo;
   g.kslabs = (a.Cin + 63) / 64;
-  g.ntaps = a.KH * a.KW;
   g.s2 = a.stride == 2 ? 1 : 0;
   g.tq = g.Tacc >= 2 ? 2 : 1;
   g.npairs = g.Tacc / g.tq;
   g.n_tiles_n = (a.Cout + 127) / 128;
   g.stack = (a.Ho <= 7 && a.Wo <= 8) ? 1 : 0;
-  g.flat = (g.ntaps == 1 && !g.stack && a.Ho >= 16) ? 1 : 0;
-  g.pw = g.flat ? 8 : kPW;
-  g.row_bytes = g.pw * 128;
-  g.halo_t = g.pw * kPH * 128;
-  g.tile_rows = g.flat ? 16 : kTileRows;
-  g.row_tiles = (a.Ho + g.tile_rows - 1) / g.tile_rows;
+  g.row_tiles = (a.Ho + kTileRows - 1) / kTileRows;
   g.w_strips = (a.Wo + 7) / 8;
   g.tmem_cols = g.npairs >= 2 ? 512 : (g.tq == 2 ? 256 : 128);
   g.lif = a.lif;
@@ -932,7 +923,7 @@ int launch(const ConvArgs &a, cudaStream_t stream) {
                             (cuuint64_t)a.B, (cuuint64_t)g.Tacc};
       cuuint64_t strides[4] = {(cuuint64_t)s_ * a.Cin * es, (cuuint64_t)s_ * a.W * a.Cin * es, (cuuint64_t)a.H * a.W * a.Cin * es,
                                g.Tacc > 1 ? (cuuint64_t)a.x_t_stride * es : frame_bytes};
-      cuuint32_t box[5] = {64, (cuuint32_t)g.pw, (cuuint32_t)(g.stack ? 9 : kPH), 1, 1};
+      cuuint32_t box[5] = {64, kPW, (cuuint32_t)(g.stack ? 9 : kPH), 1, 1};
       const char *base = static_cast<const char *>(a.x) + ((size_t)pa * a.W + pb) * a.Cin * es;
       const int rc = encode_tmap(&xph[ph], a.dtype, 5, base, dims, strides, box);
       if (rc != SNNB_OK) return rc;
@@ -941,14 +932,14 @@ int launch(const ConvArgs &a, cudaStream_t stream) {
     if (!g.s2) xph[1] = xph[2] = xph[3] = xm;
   }
   {
-    const cuuint64_t K = (cuuint64_t)g.ntaps * a.Cin;
+    const cuuint64_t K = (cuuint64_t)9 * a.Cin;
     cuuint64_t dims[2] = {K, (cuuint64_t)a.Cout};
     cuuint64_t strides[1] = {K * es};
     cuuint32_t box[2] = {64, 128};
     const int rc = encode_tmap(&wm, a.dtype, 2, a.w, dims, strides, box);
     if (rc != SNNB_OK) return rc;
   }
-  g.twin = (a.Cout <= 64 && g.ntaps == 9 && !g.s2 && !g.stack && g.sc_slabs == 0 && twin_enabled()) ? 1 : 0;
+  g.twin = (a.Cout <= 64 && !g.s2 && !g.stack && g.sc_slabs == 0 && twin_enabled()) ? 1 : 0;
   g.dup = (a.Cout <= 64 && !g.twin) ? 1 : 0;
   g.stage_off = 0;
   g.own = (a.lif && a.v_init != nullptr && a.v_init == a.v_out) ? 1 : 0;
@@ -957,7 +948,7 @@ int launch(const ConvArgs &a, cudaStream_t stream) {
   consume_wait_selftest(&g.wait_limit, &g.drop_load);
   CUtensorMap wm64 = wm;
   if (g.dup || g.twin) {
-    const cuuint64_t K = (cuuint64_t)g.ntaps * a.Cin;
+    const cuuint64_t K = (cuuint64_t)9 * a.Cin;
     cuuint64_t dims[2] = {K, (cuuint64_t)a.Cout};
     cuuint64_t strides[1] = {K * es};
     cuuint32_t box[2] = {64, (cuuint32_t)(g.twin ? 32 : 64)};
@@ -971,7 +962,7 @@ int launch(const ConvArgs &a, cudaStream_t stream) {
     cuuint64_t dims[5] = {sC, (cuuint64_t)a.Wo, (cuuint64_t)a.Ho, (cuuint64_t)a.B, (cuuint64_t)a.T};
     cuuint64_t strides[4] = {s_ * sC * es, s_ * (cuuint64_t)a.sc_W * sC * es, (cuuint64_t)a.sc_H * a.sc_W * sC * es,
                              (cuuint64_t)a.sc_t_stride * es};
-    cuuint32_t box[5] = {64, (cuuint32_t)g.pw, (cuuint32_t)(g.stack ? 9 : kPH), 1, 1};
+    cuuint32_t box[5] = {64, kPW, (cuuint32_t)(g.stack ? 9 : kPH), 1, 1};
     int rc = encode_tmap(&rm, a.dtype, 5, a.sc_x, dims, strides, box);
     if (rc != SNNB_OK) return rc;
     cuuint64_t wdims[2] = {sC, (cuuint64_t)a.Cout};
@@ -983,21 +974,21 @@ int launch(const ConvArgs &a, cudaStream_t stream) {
     cuuint64_t dims[5] = {(cuuint64_t)a.Cout, (cuuint64_t)a.Wo, (cuuint64_t)a.Ho, (cuuint64_t)a.B, (cuuint64_t)a.T};
     cuuint64_t strides[4] = {(cuuint64_t)a.Cout * es, (cuuint64_t)a.Wo * a.Cout * es, (cuuint64_t)a.Ho * a.Wo * a.Cout * es,
                              (cuuint64_t)a.B * a.Ho * a.Wo * a.Cout * es};
-    cuuint32_t box[5] = {64, (cuuint32_t)g.pw, (cuuint32_t)(g.stack ? 9 : kPH), 1, 1};
+    cuuint32_t box[5] = {64, kPW, (cuuint32_t)(g.stack ? 9 : kPH), 1, 1};
     const int rc = encode_tmap(&rm, a.dtype, 5, a.res, dims, strides, box);
     if (rc != SNNB_OK) return rc;
   }
   // [identity block] + weight ring + halo ring + room for the junk rows the last descriptor group reads past a slot
-  g.ring = g.flat ? kPairRingMax : kPairRing;
+  g.ring = kPairRing;
   const bool ident = g.has_res && !g.sc_slabs;
   g.wring = ident ? kWRingP - 1 : kWRingP;
-  size_t smem = (ident ? (size_t)kIdentBytes : 0) + (size_t)g.wring * kWSlot + (size_t)g.ring * g.tq * g.halo_t +
+  size_t smem = (ident ? (size_t)kIdentBytes : 0) + (size_t)g.wring * kWSlot + (size_t)g.ring * g.tq * kHaloT +
                 4 * kRowBytes + 1024;
   g.wres = 0;
   if (g.twin) {   // a smaller identity block and weight ring make room for the exchange buffers
     g.wring = ident ? 3 : 4;
     // (the junk rows read past the last halo slot fall into the exchange buffers, which only the epilogue writes)
-    g.stage_off = (ident ? kTwinIdentBytes : 0) + g.wring * kWSlot + g.ring * g.tq * g.halo_t;
+    g.stage_off = (ident ? kTwinIdentBytes : 0) + g.wring * kWSlot + g.ring * g.tq * kHaloT;
     smem = (size_t)g.stage_off + kXchgBytes + 1024;
     static_assert(kTwinIdentBytes + 3 * kWSlot + kPairRing * 2 * kHaloT + kXchgBytes + 1024 <= 225 * 1024, "twin mode: shared memory");
     static_assert(4 * kWSlot + kPairRing * 2 * kHaloT + kXchgBytes + 1024 <= 225 * 1024, "twin mode: shared memory");
@@ -1005,7 +996,7 @@ int launch(const ConvArgs &a, cudaStream_t stream) {
       g.wres = 1;
       g.wring = 6;
       g.ring = 2;
-      g.stage_off = g.wring * kWSlot + g.ring * g.tq * g.halo_t;
+      g.stage_off = g.wring * kWSlot + g.ring * g.tq * kHaloT;
       smem = (size_t)g.stage_off + kXchgBytes + 1024;
       static_assert(6 * kWSlot + 2 * 2 * kHaloT + kXchgBytes + 1024 <= 225 * 1024, "twin mode, resident weights: shared memory");
       static_assert(6 <= kWBarsP, "twin mode, resident weights: barriers");

@@ -439,7 +439,10 @@ extern "C" int snnb_device_status(int *status_out) {
   int h6 = 0;
   const int rc6 = split_device_status(&h6);
   if (rc6 != SNNB_OK) return rc6;
-  *status_out = h | h2 | h3 | h4 | h5 | h6;
+  int h7 = 0;
+  const int rc7 = pw_device_status(&h7);
+  if (rc7 != SNNB_OK) return rc7;
+  *status_out = h | h2 | h3 | h4 | h5 | h6 | h7;
   return SNNB_OK;
 }
 
