@@ -92,10 +92,18 @@ class Gate:
 
 def is_nhwc_dense(t: torch.Tensor) -> bool:
     """True if a [..., C, H, W] tensor is stored densely with C innermost ([..., H, W, C] memory)."""
-    if t.dim() < 4:
+    shape, stride = t.shape, t.stride()
+    d = len(shape)
+    if d < 4:
         return False
-    perm = list(range(t.dim() - 3)) + [t.dim() - 2, t.dim() - 1, t.dim() - 3]
-    return t.permute(perm).is_contiguous()
+    expect = 1
+    for i in (d - 3, d - 1, d - 2, *range(d - 4, -1, -1)):   # innermost to outermost; a size of 1 has no stride
+        n = shape[i]
+        if n != 1:
+            if stride[i] != expect:
+                return 0 in shape
+            expect *= n
+    return True
 
 
 def to_nhwc(t: torch.Tensor) -> torch.Tensor:
@@ -110,12 +118,12 @@ def to_nhwc(t: torch.Tensor) -> torch.Tensor:
 
 def empty_nhwc(shape: Sequence[int], dtype, device) -> torch.Tensor:
     """Uninitialised logical [..., C, H, W] tensor with channels-last memory."""
-    shape = list(shape)
-    lead = len(shape) - 3
-    c, h, w = shape[lead:]
-    base = torch.empty(shape[:lead] + [h, w, c], dtype=dtype, device=device)
-    inv = list(range(lead)) + [lead + 2, lead, lead + 1]
-    return base.permute(inv)
+    *lead, c, h, w = shape
+    strides, step = [1, w * c, c], h * w * c
+    for n in reversed(lead):
+        strides.insert(0, step)
+        step *= n
+    return torch.empty_strided((*lead, c, h, w), strides, dtype=dtype, device=device)
 
 
 def state_or_none(v_init: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
@@ -134,18 +142,18 @@ def stack_frames(xs: Sequence[torch.Tensor]) -> Tuple[torch.Tensor, int, bool]:
     """
     first = xs[0]
     T = len(xs)
-    if all(x.data_ptr() == first.data_ptr() for x in xs) and is_nhwc_dense(first):
-        return first, 0, False
-    if all(is_nhwc_dense(x) for x in xs):
-        if T == 1:
+    ptrs = [x.data_ptr() for x in xs]
+    same = ptrs.count(ptrs[0]) == T
+    if is_nhwc_dense(first):
+        if same:
             return first, 0, False
-        esz = first.element_size()
-        step = xs[1].data_ptr() - first.data_ptr()
-        if step > 0 and step % esz == 0 and all(
-            xs[t].data_ptr() - first.data_ptr() == t * step for t in range(T)
-        ) and step // esz >= first.numel():
+        stride, esz = first.stride(), first.element_size()
+        step = ptrs[1] - ptrs[0]
+        if (step > 0 and step % esz == 0 and step // esz >= first.numel()
+                and ptrs == list(range(ptrs[0], ptrs[0] + T * step, step))
+                and all(x.stride() == stride or is_nhwc_dense(x) for x in xs)):
             return first, step // esz, False
-    if all(x.data_ptr() == first.data_ptr() for x in xs):
+    if same:
         return to_nhwc(first), 0, True
     out = empty_nhwc([T] + list(first.shape), first.dtype, first.device)
     for t, x in enumerate(xs):

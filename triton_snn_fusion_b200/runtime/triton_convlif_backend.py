@@ -209,8 +209,8 @@ def _launch(x_base, x_t_stride, T, weight, bias, residual, v_init, stride, paddi
             spikes, v_next, lif=True, spike_dtype=None, v_dtype=None, t0=0):
     """One C-ABI call over timesteps t0 .. t0 + T - 1. x_base: [B,Cin,H,W] channels-last frame 0; ``residual`` and
     ``spikes`` are dense channels-last stacks whose frame t0 is where this call starts."""
-    B, Cin, H, W = (int(d) for d in x_base.shape)
-    Cout, _, KH, KW = (int(d) for d in weight.shape)
+    B, Cin, H, W = x_base.shape
+    Cout, _, KH, KW = weight.shape
     s = as_pair(stride)[0]
     p = as_pair(padding)[0]
     th, vr, ta = lif_scalars(v_threshold, v_reset, tau)
@@ -300,6 +300,13 @@ def _check_list(xs, what, reasons):
         reasons.append(f"{what} must be a non-empty list/tuple of tensors")
         return
     first = xs[0]
+    if isinstance(first, torch.Tensor):
+        shape, dtype, device = first.shape, first.dtype, first.device
+        for x in xs:
+            if not isinstance(x, torch.Tensor) or x.shape != shape or x.dtype != dtype or x.device != device:
+                break
+        else:
+            return
     for i, x in enumerate(xs):
         if not isinstance(x, torch.Tensor):
             reasons.append(f"{what}[{i}] is not a tensor")
@@ -308,6 +315,40 @@ def _check_list(xs, what, reasons):
             reasons.append(f"{what}[{i}] shape {tuple(x.shape)} differs from first shape {tuple(first.shape)}")
         if x.device != first.device or x.dtype != first.dtype:
             reasons.append(f"{what}[{i}] device/dtype differs from first tensor")
+
+
+# What a call's shapes, types and options alone decide: its kernel key and output shape, by those plain values. Only calls
+# that passed every check of check_triton_support are kept, oldest out first.
+_PLANS: "OrderedDict[tuple, tuple]" = OrderedDict()
+_PLANS_MAX = 1024
+
+
+def _plan(x, weight, bias, v_init, stride, padding, dilation, groups, v_threshold, v_reset, tau, detach_reset, strict, verbose):
+    """(kernel key, output shape [B, C, H, W]) of a call, after the checks; raises what they find."""
+    stride, padding, dilation, groups = as_pair(stride), as_pair(padding), as_pair(dilation), int(groups)
+    sig = None
+    if (isinstance(x, torch.Tensor) and isinstance(weight, torch.Tensor) and isinstance(bias, torch.Tensor)
+            and isinstance(v_init, torch.Tensor) and float(tau) != 0.0):
+        sig = (x.shape, x.dtype, x.device, weight.shape, weight.dtype, weight.device, bias.shape, bias.dtype, bias.device,
+               v_init.shape, v_init.dtype, v_init.device, stride, padding, dilation, groups)
+        hit = _PLANS.get(sig)
+        if hit is not None:
+            return hit
+    reasons = check_triton_support(x, weight, bias, v_init, stride, padding, dilation, groups, v_threshold, v_reset, tau,
+                                   detach_reset)
+    raise_reasons("temporal_conv", reasons, strict, verbose)
+    key = classify_conv_lif_config(weight, stride, padding, dilation, groups)
+    if key == "unsupported":
+        raise RuntimeError("unsupported dispatch key after support check")
+    plan = (key, _conv2d_output_shape(x, weight, stride, padding, dilation))
+    if sig is not None:
+        _PLANS[sig] = plan
+        if len(_PLANS) > _PLANS_MAX:
+            try:
+                _PLANS.popitem(last=False)
+            except KeyError:
+                pass   # another thread was quicker
+    return plan
 
 
 def _run_temporal(kind, xs, residuals, weight, bias, v_init, stride, padding, dilation, groups,
@@ -322,14 +363,10 @@ def _run_temporal(kind, xs, residuals, weight, bias, v_init, stride, padding, di
             reasons.append(f"xs and residuals length mismatch: {len(xs)} vs {len(residuals)}")
     raise_reasons("temporal_conv", reasons, strict, verbose)
     first = x_seq[0] if x_seq is not None else xs[0]
-    reasons = check_triton_support(first, weight, bias, v_init, stride, padding, dilation, groups,
-                                   v_threshold, v_reset, tau, detach_reset)
-    raise_reasons("temporal_conv", reasons, strict, verbose)
+    key, out_shape = _plan(first, weight, bias, v_init, stride, padding, dilation, groups, v_threshold, v_reset, tau,
+                           detach_reset, strict, verbose)
     if compute_dtype is not None and compute_dtype not in ("float32", "float16", "bfloat16"):
         raise RuntimeError(f"compute_dtype={compute_dtype} is not a known dtype path")
-    key = classify_conv_lif_config(weight, stride, padding, dilation, groups)
-    if key == "unsupported":
-        raise RuntimeError("unsupported dispatch key after support check")
     if kind is not None:
         _validate_kind(kind, key)
     if verbose:
@@ -342,14 +379,13 @@ def _run_temporal(kind, xs, residuals, weight, bias, v_init, stride, padding, di
         x_base, x_stride = xq[0], (xq.stride(0) if T > 1 else 0)
     else:
         T = len(xs)
-        x_base, x_stride, copied = stack_frames(list(xs))
-    _, cout, ho, wo = _conv2d_output_shape(first, weight, stride, padding, dilation)
-    B = int(first.shape[0])
+        x_base, x_stride, copied = stack_frames(xs)
+    B, cout, ho, wo = out_shape
     res_base = None
     if residuals is not None:
-        if tuple(residuals[0].shape) != (B, cout, ho, wo):
+        if residuals[0].shape != out_shape:
             raise RuntimeError(f"residual shape {tuple(residuals[0].shape)} does not match conv output {(B, cout, ho, wo)}")
-        r_base, r_stride, r_copied = stack_frames(list(residuals))
+        r_base, r_stride, r_copied = stack_frames(residuals)
         if T > 1 and r_stride != r_base.numel():
             stacked = empty_nhwc([T, B, cout, ho, wo], first.dtype, first.device)
             for t, r in enumerate(residuals):

@@ -50,20 +50,18 @@ def check_temporal_lif_support(x_seq, v_init, v_threshold, v_reset, tau, detach_
 
 def _same_dense_layout(x_seq: torch.Tensor, v: Optional[torch.Tensor]) -> bool:
     """x_seq[t] frames densely packed, T outermost, and v (if any) laid out like one frame."""
-    T = int(x_seq.shape[0])
-    frame = x_seq[0]
-    n = frame.numel()
-    if T > 1 and x_seq.stride(0) != n:
+    T, *frame = x_seq.shape
+    t_stride, *strides = x_seq.stride()
+    if T > 1 and t_stride * T != x_seq.numel():
         return False
     # dense and non-overlapping within a frame: sorted strides must tile the frame exactly
-    dims = sorted(((s, d) for s, d in zip(frame.stride(), frame.shape) if d > 1))
     expect = 1
-    for s, d in dims:
+    for s, d in sorted((s, d) for s, d in zip(strides, frame) if d > 1):
         if s != expect:
             return False
         expect *= d
     if v is not None:
-        return all(sv == sf for sv, sf, d in zip(v.stride(), frame.stride(), frame.shape) if d > 1)
+        return all(sv == sf for sv, sf, d in zip(v.stride(), strides, frame) if d > 1)
     return True
 
 
@@ -97,7 +95,7 @@ def run_triton_fused_temporal_lif_state(
         x_seq = x_seq.contiguous()
         v0 = v0.contiguous() if v0 is not None else None
     T = int(x_seq.shape[0])
-    n = x_seq[0].numel()
+    n = x_seq.numel() // T
     s_dt = spike_dtype or x_seq.dtype
     v_dt = v_dtype or x_seq.dtype
     spikes = torch.empty_strided(x_seq.shape, x_seq.stride(), dtype=s_dt, device=x_seq.device)
