@@ -359,3 +359,37 @@ def test_conv3x3_few_output_channels(cout, T, soft):
     ref = orc.temporal_conv_only([orc.widen(x) for x in xs], orc.widen(w), orc.widen(b), [1, 1], [1, 1])
     out = _conv_be().conv_bias_only([x.to(DEV) for x in xs], w.to(DEV), b.to(DEV), [1, 1], [1, 1])
     torch.testing.assert_close(out.cpu().float(), ref, rtol=1e-2, atol=1e-2)
+
+
+@pytest.mark.parametrize("case", [
+    # T, B, cin, cout, k, stride, H, W: channel counts and T whose accumulators do not fit tensor memory at full width
+    (5, 2, 64, 112, 3, 1, 9, 10),     # 5 x 112 columns: tiles of 48 (odd T: the halo kernel by default)
+    (7, 1, 128, 80, 3, 1, 16, 9),     # 32
+    (11, 2, 64, 48, 3, 1, 8, 8),      # 16
+    (12, 1, 64, 112, 3, 2, 17, 12),   # 48, then 16
+    (8, 2, 64, 80, 5, 1, 10, 9),      # no kernel but the general one takes a 5x5 window
+    (32, 1, 64, 16, 1, 2, 9, 9),      # the narrowest tile at the longest T
+])
+def test_channel_tiles_that_are_halved_for_many_timesteps(case):
+    T, B, cin, cout, k, s, H, W = case
+    dtype = torch.bfloat16
+    g = torch.Generator().manual_seed(T * cout)
+    xs = [(torch.rand(B, cin, H, W, generator=g) < 0.2).to(dtype) for _ in range(T)]
+    w = (torch.randn(cout, cin, k, k, generator=g) * 2.5 / (0.2 * cin * k * k) ** 0.5).to(dtype)
+    b = (torch.randn(cout, generator=g) * 0.1).to(dtype)
+    ho, wo = (H - 1) // s + 1, (W - 1) // s + 1
+    res = (torch.rand(T, B, cout, ho, wo, generator=g) < 0.2).to(dtype)
+    v0 = (torch.randn(B, cout, ho, wo, generator=g) * 0.3).to(dtype)
+    rs, rv = orc.temporal_conv_lif([orc.widen(x) for x in xs], orc.widen(w), orc.widen(b), orc.widen(v0), [s, s], [k // 2] * 2,
+                                   [1, 1], 1, 1.0, 0.0, 2.0, residuals=[orc.widen(r) for r in res])
+    from triton_snn_fusion_b200 import _lib as L
+    be = _conv_be()
+    nhwc = lambda t: t.transpose(-3, -2).transpose(-2, -1).contiguous().to(DEV)
+    xd, wd, rd, vd, bd = nhwc(torch.stack(xs)), nhwc(w), nhwc(res), nhwc(v0), b.to(DEV)
+    sp, v = torch.empty_like(rd), torch.empty_like(vd)
+    L.check(L.lib.snnb_conv_lif(xd.data_ptr(), xd.stride(0), wd.data_ptr(), bd.data_ptr(), rd.data_ptr(), vd.data_ptr(),
+                                sp.data_ptr(), v.data_ptr(), T, B, cin, H, W, cout, k, k, s, k // 2, 1, L.BF16, L.BF16, L.BF16,
+                                1.0, 0.0, 2.0, be._PATH[be._conv_path], None), "snnb_conv_lif")
+    torch.cuda.synchronize()
+    check_parity(sp.permute(0, 1, 4, 2, 3), v.permute(0, 3, 1, 2), rs, rv, dtype, what=str(case))
+    assert 0.02 < float(rs.mean()) < 0.6

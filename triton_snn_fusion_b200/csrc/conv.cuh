@@ -33,6 +33,16 @@ struct ConvArgs {
   int sc_cin = 0, sc_H = 0, sc_W = 0, sc_stride = 1;
 };
 
+// Output-channel tile of the kernels with the channels as the MMA's N (conv_tc.cu, conv_halo.cu): `most` halved until
+// the accumulators of Tacc timesteps fit the 512 columns of tensor memory. Always a multiple of 16: N has to be one at
+// M = 128, the epilogue walks groups of 16 columns, and a tile's first channel (bias, residual, spikes) is then on a
+// 32-byte boundary. 112 channels and T = 12 are tiles of 48 and then 16, not of 56 and 28.
+inline int channel_tile(int most, int Tacc) {
+  int bn = (most + 15) / 16 * 16;
+  while (bn > 16 && Tacc * bn > 512) bn = bn / 2 < 16 ? 16 : bn / 2 / 16 * 16;
+  return bn;
+}
+
 // CUDA-core implicit GEMM (any shape, fp32 accumulate).
 int conv_lif_simt(const ConvArgs &a, cudaStream_t stream);
 

@@ -257,11 +257,7 @@ conv3x3_halo_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
   }
 }
 
-int halo_bn(int Cout, int Tacc) {
-  int bn = Cout >= 128 ? 128 : ((Cout + 15) / 16) * 16;
-  while (bn > 16 && Tacc * bn > 512) bn /= 2;
-  return bn;
-}
+int halo_bn(int Cout, int Tacc) { return channel_tile(Cout >= 128 ? 128 : Cout, Tacc); }
 
 bool fill_geom(const ConvArgs &a, HaloGeom &g) {
   g.T = a.T;

@@ -285,13 +285,8 @@ void choose_boxes(int Ho, int Wo, int &BW, int &BH, int &nbox) {
   }
 }
 
-// Output-channel tile: as wide as the T accumulators allow in the 512 TMEM columns (a wider tile
-// re-reads the activations fewer times), at most 256.
-int pick_bn(int Cout, int Tacc) {
-  int bn = Cout >= 256 ? 256 : (Cout >= 128 ? 128 : ((Cout + 15) / 16) * 16);
-  while (bn > 16 && Tacc * bn > 512) bn /= 2;
-  return bn;
-}
+// Output-channel tile: a wider tile re-reads the activations fewer times; at most 256.
+int pick_bn(int Cout, int Tacc) { return channel_tile(Cout >= 256 ? 256 : (Cout >= 128 ? 128 : Cout), Tacc); }
 
 template <typename XT, typename ST, typename VT>
 int launch(const ConvArgs &a, cudaStream_t stream) {
