@@ -331,6 +331,7 @@ def run_ours(args):
         hi, wi, _ = net.shapes[L["src"]]
         name = _lib.conv_kernel_name(T_STEPS, B, L["cin"], hi, wi, L["cout"], L["k"], L["s"], L["p"], torch.bfloat16,
                                      one_frame=(L["cin"] == 3), residual=bool(L.get("residual")))
+        name = name.split("/")[0]   # the kernel without its form
         return name + (" (3-channel stem)" if L["cin"] == 3 else "")
     by_kernel = {}
     fused_into = {D["name"]: consumer for consumer, D in net.fused_sc.items()}   # shortcut conv -> the launch it rides in

@@ -62,9 +62,10 @@ typedef enum snnb_layout { SNNB_NCHW = 0, SNNB_NHWC = 1 } snnb_layout;
  * snnb_conv_lif) and the CUDA-core path otherwise. TCGEN05 insists on a tensor-core
  * kernel (error if none applies). Among the tensor-core kernels, 3x3 / stride 1 /
  * padding 1 convs prefer the timestep-pair kernel (T = 1 or even; weights as the M
- * operand, 256 pixels as N; its form for few output tiles splits the reduction over a
- * cluster, its form for 1x1 convs and linear layers is a GEMM over the pixels, both for
- * any T), then the shared-memory halo kernel; TCGEN05_HALO skips the first, TCGEN05_TAPS forces the general one-load-per-tap kernel (for comparison). */
+ * operand, 256 pixels as N), then the shared-memory halo kernel. Before these, calls with few
+ * output tiles go to a kernel that splits the reduction over a cluster, and 1x1 convs and linear
+ * layers to a GEMM over the pixels, both for any T. TCGEN05_HALO skips all but the halo and the
+ * general kernel, TCGEN05_TAPS forces the general one-load-per-tap kernel (for comparison). */
 typedef enum snnb_path {
   SNNB_PATH_AUTO = 0, SNNB_PATH_SIMT = 1, SNNB_PATH_TCGEN05 = 2, SNNB_PATH_TCGEN05_TAPS = 3,
   SNNB_PATH_TCGEN05_HALO = 4
@@ -185,8 +186,10 @@ int snnb_conv_lif(const void *x_seq, int64_t x_t_stride, const void *w, const vo
                   float v_th, float v_reset, float tau, int path, void *stream);
 
 /*
- * Diagnostic: the name of the kernel snnb_conv_lif would run for a call of this shape ("conv3x3_pair" with its
- * forms for few tiles and for 1x1 convs, "conv3x3_halo", "conv_lif_tc", "conv3x3_smallcin" or "conv_lif_simt"), assuming 16-byte aligned dense buffers.
+ * Diagnostic: the name of the kernel snnb_conv_lif would run for a call of this shape, assuming 16-byte aligned dense
+ * buffers: "conv3x3_pair", "conv_split/S" (clusters of S), "conv_pw", "conv3x3_halo", "conv_lif_tc", "conv3x3_smallcin",
+ * "conv_lif_f32/TxN" (tiles of T steps and N channels) or "conv_lif_simt". How many clusters run at once differs between
+ * GPUs of a kind, so the choice of S, and between splitting and not, may too; without a GPU it is that of one B200.
  * one_frame != 0: the same input frame at every step (x_t_stride == 0). Launches nothing. The reference reports
  * its kernel choice through kernel_key / kernel_temporal_config of its result objects
  * (runtime/triton_convlif_backend.py:7-15); this is the C-level counterpart.

@@ -25,7 +25,7 @@ struct ConvArgs {
   // Optional shortcut branch accumulated into the same output before the LIF: a 1x1 conv with stride
   // sc_stride over a second input sc_x [T][B][sc_H][sc_W][sc_cin] (frames sc_t_stride elements apart),
   // weights sc_w [Cout][sc_cin]; its bias is folded into b by the caller. Output pixel (h, w) reads
-  // sc_x at (h * sc_stride, w * sc_stride). Only the timestep-pair kernel implements it.
+  // sc_x at (h * sc_stride, w * sc_stride). Only the timestep-pair kernel and its split form implement it.
   const void *sc_x = nullptr;
   const void *sc_w = nullptr;
   const void *b2 = nullptr;   // bias of the shortcut conv, [Cout] or null: added to b in fp32
@@ -46,8 +46,10 @@ inline int channel_tile(int most, int Tacc) {
 // CUDA-core implicit GEMM (any shape, fp32 accumulate).
 int conv_lif_simt(const ConvArgs &a, cudaStream_t stream);
 
-// The fp32 form of it with asynchronous copies and packed multiply-adds; conv_lif_simt hands it the calls it takes.
+// The fp32 form of it with asynchronous copies and packed multiply-adds.
+struct F32Tile { int TT, TN; };   // steps of a window, eighths of the channels of a block
 bool conv_f32_supported(const ConvArgs &a);
+F32Tile conv_f32_tile(const ConvArgs &a);
 int conv_f32(const ConvArgs &a, cudaStream_t stream);
 
 // Direct CUDA-core kernel for 3x3 convs over images with at most four channels (the first layer of a network).
@@ -64,11 +66,11 @@ bool conv3x3_halo_supported(const ConvArgs &a);
 int conv3x3_halo(const ConvArgs &a, cudaStream_t stream);
 int halo_device_status(int *out);
 
-// tcgen05 implicit GEMM for 3x3 (stride 1 or 2) and 1x1 convs, T = 1 or even: weights as the M operand and
+// tcgen05 implicit GEMM for 3x3 convs (stride 1 or 2), T = 1 or even: weights as the M operand and
 // the pixels of two timesteps as a 256-wide N operand (the only shape that runs the tensor pipe at
 // its full rate), halo tiles in shared memory. Preferred over conv3x3_halo when supported.
 bool conv3x3_pair_supported(const ConvArgs &a);
-bool pair_shape_supported(const ConvArgs &a);   // all of it but the number of timesteps
+bool pair_shape_supported(const ConvArgs &a);   // the shapes of its tiles, any T; 1x1 too, for conv_split.cu
 int conv3x3_pair(const ConvArgs &a, cudaStream_t stream);
 int pair_device_status(int *out);
 // The form of it for 1x1 convs and linear layers, any T (conv_pw.cu).
@@ -76,12 +78,12 @@ bool conv_pw_supported(const ConvArgs &a);
 int conv_pw(const ConvArgs &a, cudaStream_t stream);
 int pw_device_status(int *out);
 // The form of it for calls with few output tiles (conv_split.cu): the reduction of a tile over a cluster of CTAs.
-// conv_split_plan returns the cluster size, 0 where the timestep-pair kernel itself is the better one.
+// conv_split_plan returns the cluster size, 0 where whole tiles are the better choice.
 int conv_split_plan(const ConvArgs &a);
 int conv_split(const ConvArgs &a, int S, cudaStream_t stream);
 int split_device_status(int *out);
 // Self-test of the bounded waits (snnb_selftest_arm_wait_timeout): if armed, hands the shortened limit and the
-// "drop one load" switch to the next launch of the timestep-pair kernel and disarms.
+// "drop one load" switch to the next launch of the timestep-pair, split or 1x1 kernel and disarms.
 void consume_wait_selftest(long long *limit_cycles, int *drop_load);
 
 // GEMM + LIF stage of the 7x7 / stride 2 stem on the re-laid image (stem.cu): persistent tcgen05 kernel

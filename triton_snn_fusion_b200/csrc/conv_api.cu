@@ -15,22 +15,39 @@ bool membranes_overlap_partially(const ConvArgs &a) {
   return p < q + bytes && q < p + bytes;
 }
 
+enum class Kernel { smallcin, simt, f32, split, pw, pair, halo, taps, none };
+
+// The kernel of a call. `S`: cluster size of the split kernel; `why`: what keeps a call with none off the tensor cores.
+Kernel choose(const ConvArgs &a, int path, int *S, const char **why) {
+  const Kernel cuda_cores = conv_f32_supported(a) ? Kernel::f32 : Kernel::simt;
+  if (path == SNNB_PATH_AUTO && conv_smallcin_supported(a)) return Kernel::smallcin;   // RGB first layers
+  if (path == SNNB_PATH_SIMT) return cuda_cores;
+  if (path != SNNB_PATH_TCGEN05_TAPS && path != SNNB_PATH_TCGEN05_HALO) {
+    if ((*S = conv_split_plan(a)) != 0) return Kernel::split;
+    if (conv_pw_supported(a)) return Kernel::pw;
+    if (conv3x3_pair_supported(a)) return Kernel::pair;
+  }
+  if (path != SNNB_PATH_TCGEN05_TAPS && conv3x3_halo_supported(a)) return Kernel::halo;
+  if (conv_lif_tc_supported(a, why)) return Kernel::taps;
+  return path == SNNB_PATH_AUTO ? cuda_cores : Kernel::none;
+}
+
 int run(const ConvArgs &a, int path, cudaStream_t stream, const char *what) {
   if (membranes_overlap_partially(a))
     return fail(SNNB_ERR_INVALID, "%s: v_init and v_out overlap without being the same buffer", what);
-  if (path == SNNB_PATH_AUTO && conv_smallcin_supported(a)) return conv_smallcin(a, stream);   // RGB first layers
-  if (path == SNNB_PATH_SIMT) return conv_lif_simt(a, stream);
-  const bool taps_only = path == SNNB_PATH_TCGEN05_TAPS;
-  if (!taps_only && path != SNNB_PATH_TCGEN05_HALO) {
-    if (const int S = conv_split_plan(a)) return conv_split(a, S, stream);
-    if (conv_pw_supported(a)) return conv_pw(a, stream);
-  }
-  if (!taps_only && path != SNNB_PATH_TCGEN05_HALO && conv3x3_pair_supported(a)) return conv3x3_pair(a, stream);
-  if (!taps_only && conv3x3_halo_supported(a)) return conv3x3_halo(a, stream);
+  int S = 0;
   const char *why = "";
-  if (conv_lif_tc_supported(a, &why)) return conv_lif_tc(a, stream);
-  if (path == SNNB_PATH_AUTO) return conv_lif_simt(a, stream);
-  return fail(SNNB_ERR_UNSUPPORTED, "%s: tcgen05 path not available for this call: %s", what, why);
+  switch (choose(a, path, &S, &why)) {
+    case Kernel::smallcin: return conv_smallcin(a, stream);
+    case Kernel::simt: return conv_lif_simt(a, stream);
+    case Kernel::f32: return conv_f32(a, stream);
+    case Kernel::split: return conv_split(a, S, stream);
+    case Kernel::pw: return conv_pw(a, stream);
+    case Kernel::pair: return conv3x3_pair(a, stream);
+    case Kernel::halo: return conv3x3_halo(a, stream);
+    case Kernel::taps: return conv_lif_tc(a, stream);
+    default: return fail(SNNB_ERR_UNSUPPORTED, "%s: tcgen05 path not available for this call: %s", what, why);
+  }
 }
 
 }  // namespace
@@ -83,15 +100,28 @@ extern "C" int snnb_conv_lif_which(int T, int B, int Cin, int H, int W, int Cout
   a.x_t_stride = one_frame ? 0 : (int64_t)B * H * W * Cin;
   a.lif = lif ? 1 : 0; a.dtype = dtype; a.spike_dtype = dtype; a.v_dtype = dtype;
   a.p = make_lif_params(1.0f, 0.0f, 2.0f);
-  const char *k = "conv_lif_simt";
-  const bool taps_only = path == SNNB_PATH_TCGEN05_TAPS;
-  const char *why = "";
-  if (path == SNNB_PATH_AUTO && conv_smallcin_supported(a)) k = "conv3x3_smallcin";
-  else if (path == SNNB_PATH_SIMT) k = "conv_lif_simt";
-  else if (!taps_only && path != SNNB_PATH_TCGEN05_HALO && (conv3x3_pair_supported(a) || conv_pw_supported(a) || conv_split_plan(a))) k = "conv3x3_pair";
-  else if (!taps_only && conv3x3_halo_supported(a)) k = "conv3x3_halo";
-  else if (conv_lif_tc_supported(a, &why)) k = "conv_lif_tc";
-  else if (path != SNNB_PATH_AUTO) return fail(SNNB_ERR_UNSUPPORTED, "conv_lif_which: no tensor-core kernel takes this call: %s", why);
+  int S = 0;
+  const char *why = "", *k = "";
+  char form[32];
+  switch (choose(a, path, &S, &why)) {
+    case Kernel::smallcin: k = "conv3x3_smallcin"; break;
+    case Kernel::simt: k = "conv_lif_simt"; break;
+    case Kernel::f32: {
+      const F32Tile t = conv_f32_tile(a);
+      snprintf(form, sizeof(form), "conv_lif_f32/%dx%d", t.TT, 8 * t.TN);
+      k = form;
+      break;
+    }
+    case Kernel::split:
+      snprintf(form, sizeof(form), "conv_split/%d", S);
+      k = form;
+      break;
+    case Kernel::pw: k = "conv_pw"; break;
+    case Kernel::pair: k = "conv3x3_pair"; break;
+    case Kernel::halo: k = "conv3x3_halo"; break;
+    case Kernel::taps: k = "conv_lif_tc"; break;
+    default: return fail(SNNB_ERR_UNSUPPORTED, "conv_lif_which: no tensor-core kernel takes this call: %s", why);
+  }
   snprintf(name, (size_t)name_len, "%s", k);
   return SNNB_OK;
 }
@@ -149,8 +179,8 @@ extern "C" int snnb_linear_lif(const void *x_seq, int64_t x_t_stride, const void
   ConvArgs a;
   a.x = x_seq; a.x_t_stride = x_t_stride; a.w = w; a.b = b; a.res = nullptr;
   a.v_init = v_init; a.spikes = spikes; a.v_out = v_out;
-  // a 1x1 conv over the tokens laid out as an image: 8 tokens per row when that divides (the shape the
-  // timestep-pair kernel tiles; at most 56 tokens are one of its whole small maps), else one row of M tokens
+  // a 1x1 conv over the tokens laid out as an image: 8 tokens per row when that divides (the shape that the split kernel
+  // tiles; at most 56 tokens are one of its whole small maps), else one row of M tokens
   const bool rows8 = M % 8 == 0;
   a.T = T; a.B = 1; a.Cin = K; a.H = rows8 ? M / 8 : 1; a.W = rows8 ? 8 : M; a.Cout = N; a.KH = 1; a.KW = 1;
   a.stride = 1; a.pad = 0; a.Ho = a.H; a.Wo = a.W; a.lif = 1;

@@ -7,8 +7,8 @@
 //  * Rows = pixels x TT timesteps. A thread's eight rows are TT consecutive steps of 8 / TT pixels, so the LIF of a
 //    pixel runs inside one thread straight from the accumulators, the weights staged for a tile serve all TT steps, and
 //    a layer has T times as many tiles' worth of rows to spread over the SMs (16 x 16 maps, batch 16, 128 channels:
-//    256 blocks). Longer sequences walk windows of TT steps with the membrane in shared memory (pick_tile). One frame for all steps (direct encoding) is convolved once (TT = 1) and its LIF
-//    repeated.
+//    256 blocks). Longer sequences walk windows of TT steps with the membrane in shared memory (pick_tile). One frame
+//    for all steps (direct encoding) is convolved once (TT = 1) and its LIF repeated.
 //  * Both operands keep K contiguous in shared memory (what 16-byte cp.async delivers, with zero fill for padding, the
 //    last K chunk and rows past the end), rows 20 words apart: the 16-byte fragment reads of eight neighbouring rows
 //    touch all 32 banks once.
@@ -254,7 +254,6 @@ int launch_f32(const ConvArgs &a, const F32Geom &g, cudaStream_t stream) {
 // batch 16, 128 -> 128 channels, T = 4: predicted 2.0 / 2.4 / 2.3 / 4.0 for (steps, channels) = (4, 64) / (4, 32) /
 // (2, 64) / (8, 64), measured 152 / 182 / 188 / 276 us. Odd T is rounded up to whole windows by the same estimate:
 // T = 3, 28 x 28, 512 -> 1024 takes 756 us with a window of four, 932 us with three windows of one.
-struct F32Tile { int TT, TN; };
 F32Tile pick_tile(const F32Geom &g) {
   const int sms = sm_count() > 0 ? sm_count() : 148;
   F32Tile best = {1, 8};
@@ -299,7 +298,8 @@ bool conv_f32_supported(const ConvArgs &a) {
          (128 / ((long long)a.Ho * a.Wo) + 2) * a.H * a.W * a.Cin < (1LL << 31) && !a.xs_w && !a.xs_h && !a.xs_b && !a.xd_w && !a.xd_h && a.sc_x == nullptr;
 }
 
-int conv_f32(const ConvArgs &a, cudaStream_t stream) {
+namespace {
+F32Geom make_geom(const ConvArgs &a) {
   F32Geom g;
   g.T = a.T; g.nwin = 1; g.Cin = a.Cin; g.H = a.H; g.W = a.W; g.Cout = a.Cout; g.KH = a.KH; g.KW = a.KW;
   g.stride = a.stride; g.pad = a.pad; g.Ho = a.Ho; g.Wo = a.Wo; g.K = a.KH * a.KW * a.Cin; g.lif = a.lif;
@@ -308,6 +308,14 @@ int conv_f32(const ConvArgs &a, cudaStream_t stream) {
   g.M = (long long)a.B * a.Ho * a.Wo;
   g.frame_out = g.M * a.Cout;
   g.vec = a.Cout % 4 == 0 && aligned16(a.spikes) && (a.res == nullptr || aligned16(a.res));
+  return g;
+}
+}  // namespace
+
+F32Tile conv_f32_tile(const ConvArgs &a) { return pick_tile(make_geom(a)); }
+
+int conv_f32(const ConvArgs &a, cudaStream_t stream) {
+  F32Geom g = make_geom(a);
   if (a.lif && a.spike_dtype == SNNB_U8) return launch_tt<uint8_t>(a, g, stream);
   return launch_tt<float>(a, g, stream);
 }

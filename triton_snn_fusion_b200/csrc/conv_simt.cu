@@ -204,7 +204,6 @@ int dispatch(const ConvArgs &a, cudaStream_t stream) {
 }  // namespace
 
 int conv_lif_simt(const ConvArgs &a, cudaStream_t stream) {
-  if (conv_f32_supported(a)) return conv_f32(a, stream);
   switch (a.dtype) {
     case SNNB_F32: return dispatch<float>(a, stream);
     case SNNB_BF16: return dispatch<__nv_bfloat16>(a, stream);
