@@ -83,3 +83,23 @@ def test_linear_with_few_tokens(T, M, K, N):
     r = be.run_triton_fused_temporal_linear_lif_state_packed(x.to(DEV), w.to(DEV), b.to(DEV),
                                                              torch.tensor(0.0, device=DEV, dtype=torch.bfloat16), 1.0, 0.0, 2.0, True)
     check_parity(r.spikes, r.v_next, rs, rv, torch.bfloat16)
+
+
+@pytest.mark.parametrize("form,B,cin,H,W", [("conv_split/8", 6, 256, 7, 7), ("conv_split/8", 5, 256, 3, 4),
+                                           ("conv_split/4", 40, 256, 7, 7), ("conv_split/8", 3, 256, 17, 13)])
+def test_an_image_comes_out_the_same_wherever_it_stands_in_the_batch(form, B, cin, H, W):
+    """Copies of one image (dense values, whose sums depend on the order of the additions) in all places of a batch, two
+    to a tile or one."""
+    from triton_snn_fusion_b200 import _lib as L
+    T, cout = 4, 128
+    assert L.conv_kernel_name(T, B, cin, H, W, cout, 3, 1, 1, torch.bfloat16).startswith("conv_split/")
+    g = torch.Generator().manual_seed(B)
+    x = torch.randn(T, 1, H, W, cin, generator=g).bfloat16().expand(T, B, H, W, cin).contiguous().to(DEV)
+    w = (torch.randn(cout, 3, 3, cin, generator=g) * 0.06).bfloat16().to(DEV)
+    b = (torch.randn(cout, generator=g) * 0.1).bfloat16().to(DEV)
+    sp, v = torch.empty(T, B, H, W, cout, dtype=torch.bfloat16, device=DEV), torch.empty(B, H, W, cout, device=DEV)
+    L.check(L.lib.snnb_conv_lif(x.data_ptr(), x.stride(0), w.data_ptr(), b.data_ptr(), None, None, sp.data_ptr(), v.data_ptr(), T, B,
+                                cin, H, W, cout, 3, 3, 1, 1, 1, L.BF16, L.BF16, L.F32, 1.0, 0.0, 2.0, L.PATH_AUTO, None), "conv")
+    for i in range(1, B):
+        assert torch.equal(v[i], v[0]) and torch.equal(sp[:, i], sp[:, 0])
+    assert 0.02 < float(sp.float().mean()) < 0.6

@@ -127,16 +127,38 @@ __device__ __forceinline__ void split_unit(const SplitGeom &g, const LifParams &
   float4 y[kMaxTw];
 #pragma unroll
   for (int q = 0; q < kMaxTw; ++q) y[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-  for (int i = 0; i < g.S; ++i, r = r + 1 == g.S ? 0 : r + 1) {
-    const uint32_t from = map_rank(src, (uint32_t)r);
-    float4 part[kMaxTw];
+  // The sum of the S partial sums, each CTA starting with its own: at any time the CTAs of a cluster read different ones
+  // (with all of them on rank 0 first the slowest took twice as long). Opposite partial sums are added first, then the sums a
+  // quarter turn apart, and so on: a + b = b + a makes that the same number wherever one starts, so a pixel that two
+  // shifted tiles compute, or an image in the other half of a tile, comes out the same.
+  const int half = g.S >> 1, quarter = g.S >> 2;
+  auto add = [](float4 &a, const float4 &b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; };
 #pragma unroll
-    for (int q = 0; q < kMaxTw; ++q)
-      if (q < tw) part[q] = ld_cluster(from + (uint32_t)q * kStageT);
+  for (int q0 = 0; q0 < kMaxTw; q0 += 2) {   // two timesteps at a time: eight loads in flight, which the registers hold
+    if (q0 < tw) {
+      const bool two = q0 + 1 < tw;
+#pragma unroll 1
+      for (int turn = 0; turn < (quarter > 1 ? 2 : 1); ++turn) {
+        float4 part[4][2];
 #pragma unroll
-    for (int q = 0; q < kMaxTw; ++q)
-      if (q < tw) { y[q].x += part[q].x; y[q].y += part[q].y; y[q].z += part[q].z; y[q].w += part[q].w; }
+        for (int i = 0; i < 4; ++i)
+          if (i < 2 || quarter) {
+            const uint32_t from = map_rank(src, (uint32_t)((r + turn + (i & 1) * half + (i >> 1) * quarter) & (g.S - 1))) + (uint32_t)q0 * kStageT;
+            part[i][0] = ld_cluster(from);
+            if (two) part[i][1] = ld_cluster(from + kStageT);
+          }
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          if (j == 0 || two) {
+            add(part[0][j], part[1][j]);
+            if (quarter) {
+              add(part[2][j], part[3][j]);
+              add(part[0][j], part[2][j]);
+            }
+            add(y[q0 + j], part[0][j]);
+          }
+      }
+    }
   }
 #pragma unroll
   for (int q = 0; q < kMaxTw; ++q)
@@ -373,17 +395,13 @@ conv_split_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
         for (int i = 0; i < 4; ++i)
           if (c_ok && col + i < g.Wo && col + i >= wlo && row >= hlo) mine |= 1 << i;
         const uint32_t src = smem_base + stage_at(0, vr, half);
-        // The order of the ranks depends on the image row alone: the CTAs of a cluster, which own different rows, read
-        // different CTAs at a time (with all of them on rank 0 first the slowest took twice as long), and a pixel that
-        // two shifted tiles compute comes out the same in both.
-        const int r0 = (row + (vr >= rows_img ? rows_img : 0)) % g.S;
         float vk[4] = {0.f, 0.f, 0.f, 0.f};
         if (win > 0) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) vk[i] = v[k][i];
         }
-        if (fast) split_unit<true>(g, p, src, r0, o, mine, vk, win, t0, tw, bias_c, res, v_init, spikes, v_out);
-        else split_unit<false>(g, p, src, r0, o, mine, vk, win, t0, tw, bias_c, res, v_init, spikes, v_out);
+        if (fast) split_unit<true>(g, p, src, rank, o, mine, vk, win, t0, tw, bias_c, res, v_init, spikes, v_out);
+        else split_unit<false>(g, p, src, rank, o, mine, vk, win, t0, tw, bias_c, res, v_init, spikes, v_out);
         if (win + 1 < g.nwin) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) v[k][i] = vk[i];
@@ -510,7 +528,7 @@ int dispatch(const ConvArgs &a, int S, cudaStream_t stream) {
 // nine 8x8 maps, T = 1: 23 against 15 / 11 / 17 (144 CTAs in clusters of eight do not fit at once); 128 -> 128 stride 2 to
 // 7x7, 116 images: 29 against 37 with S = 2. Split only for a clear gain (a tenth).
 // A sum over S partial sums rounds elsewhere than the pair kernel's chain, so outputs of a small batch agree with those of
-// a large one to fp32 rounding of the currents, not always bit for bit.
+// a large one to fp32 rounding of the currents, not always bit for bit. Within a batch an image's place does not matter.
 int conv_split_plan(const ConvArgs &a) {
   if (!pair_shape_supported(a) || a.T > 64) return 0;
   const bool stack = a.Ho <= 7 && a.Wo <= 8;
