@@ -52,3 +52,21 @@ def test_kernel_choice_is_reported_without_a_gpu():
     import pytest
     with pytest.raises(_lib.SnnbError, match="no tensor-core kernel"):
         name(4, 8, 24, 13, 11, 40, 5, 1, 2, bf, path=_lib.PATH_TCGEN05)
+
+
+def test_kernel_choice_of_calls_with_few_tiles_and_of_1x1_convs():
+    """The lines that the dispatch draws between the split kernel and those that compute whole tiles, with the
+    cluster counts of the B200 that they were measured on (15 and 33 clusters of 8 and 4 at a time)."""
+    import pytest
+    import torch
+    from triton_snn_fusion_b200 import _lib
+    if torch.cuda.is_available():
+        pytest.skip("the cluster counts are those of the GPU at hand")
+    bf, name = torch.bfloat16, _lib.conv_kernel_name
+    assert name(4, 1, 512, 7, 7, 512, 3, 1, 1, bf) == "conv_split/8"
+    assert name(6, 2, 128, 11, 11, 488, 3, 1, 1, bf) != "conv_split/8"       # 16 tiles: one cluster of eight too many
+    assert name(4, 8, 512, 7, 7, 512, 3, 1, 1, bf) == "conv_split/4"
+    assert name(4, 3, 384, 31, 31, 24, 3, 1, 1, bf) == "conv3x3_pair"        # 36 tiles do not fit at S = 4
+    assert name(3, 8, 192, 9, 9, 24, 3, 1, 1, bf).startswith("conv_split/")  # odd T, 24 channels: nothing else takes it
+    assert name(8, 1, 640, 15, 8, 48, 1, 1, 0, bf) == "conv_pw"              # two windows for ten weight tiles do not pay
+    assert name(12, 14, 1408, 1, 1, 72, 1, 1, 0, bf) == "conv_split/8"

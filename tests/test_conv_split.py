@@ -9,28 +9,34 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 CASES = [
-    # T, B, cin, cout, k, stride, H, W, residual, carried state
-    (4, 1, 512, 512, 3, 1, 7, 7, True, False),     # one image in a tile that holds two
-    (4, 3, 256, 200, 3, 1, 7, 7, True, True),      # two images and one; the last channel tile is ragged
-    (4, 1, 256, 512, 3, 2, 14, 14, False, False),  # stride 2: four phase tiles per slab
-    (4, 2, 256, 128, 3, 2, 29, 31, True, True),    # odd strided map, last tiles shifted back inside the image
-    (1, 2, 256, 256, 3, 1, 8, 8, False, True),     # one step
-    (3, 1, 256, 256, 3, 1, 13, 11, True, True),    # odd T: a pair and a single step in one window
-    (6, 1, 256, 128, 3, 1, 16, 9, True, True),     # windows of four and two steps
-    (7, 1, 384, 128, 3, 1, 15, 8, False, False),   # windows of four and three
-    (4, 1, 1152, 136, 1, 1, 14, 14, False, True),  # 1x1, ragged channels out
-    (2, 1, 1160, 256, 1, 1, 9, 8, False, False),   # 1x1, the last slab is partly filled
-    (12, 1, 512, 128, 3, 1, 5, 3, True, False),    # three windows, map smaller than half a tile row
+    # cluster size; T, B, cin, cout, k, stride, H, W, residual, carried state
+    (8, 4, 1, 512, 512, 3, 1, 7, 7, True, False),     # one image in a tile that holds two
+    (8, 4, 3, 256, 200, 3, 1, 7, 7, True, True),      # two images and one; the last channel tile is ragged
+    (8, 4, 1, 256, 512, 3, 2, 14, 14, False, False),  # stride 2: four phase tiles per slab
+    (8, 4, 2, 256, 128, 3, 2, 29, 31, True, True),    # odd strided map, last tiles shifted back inside the image
+    (8, 1, 2, 256, 256, 3, 1, 8, 8, False, True),     # one step
+    (8, 3, 1, 256, 256, 3, 1, 13, 11, True, True),    # odd T: a pair and a single step in one window
+    (8, 6, 1, 256, 128, 3, 1, 16, 9, True, True),     # windows of four and two steps
+    (8, 7, 1, 384, 128, 3, 1, 15, 8, False, False),   # windows of four and three
+    (8, 4, 1, 1152, 136, 1, 1, 14, 14, False, True),  # 1x1, ragged channels out
+    (8, 2, 1, 1160, 256, 1, 1, 9, 8, False, False),   # 1x1, the last slab is partly filled
+    (8, 12, 1, 512, 128, 3, 1, 5, 3, True, False),    # three windows, map smaller than half a tile row
+    (4, 6, 24, 192, 100, 3, 1, 8, 8, True, True),        # windows of four and two steps
+    (4, 3, 9, 256, 256, 3, 1, 9, 8, True, True),         # odd T
+    (4, 4, 21, 1024, 256, 1, 1, 7, 8, False, True),      # 1x1, two images per tile and one
+    (2, 1, 4, 512, 512, 3, 1, 16, 16, True, True),       # a CTA owns seven rows, all that its warps have room for
+    (2, 4, 99, 512, 128, 3, 1, 7, 7, True, False),       # the same with two images per tile and one
+    (2, 5, 40, 512, 128, 3, 1, 8, 8, False, True),       # windows of four steps and one
 ]
 
 
 @pytest.mark.parametrize("case", CASES)
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_against_the_oracle(case, dtype):
-    T, B, cin, cout, k, s, H, W, residual, carry = case
+    S, T, B, cin, cout, k, s, H, W, residual, carry = case
     from triton_snn_fusion_b200 import _lib
     from triton_snn_fusion_b200.runtime import triton_convlif_backend as be
-    assert _lib.conv_kernel_name(T, B, cin, H, W, cout, k, s, k // 2, dtype, residual=residual).startswith("conv_split/")
+    assert _lib.conv_kernel_name(T, B, cin, H, W, cout, k, s, k // 2, dtype, residual=residual) == f"conv_split/{S}"
     g = torch.Generator().manual_seed(T * 1000 + cin + cout)
     xs = [(torch.rand(B, cin, H, W, generator=g) < 0.2).to(dtype) for _ in range(T)]
     w = (torch.randn(cout, cin, k, k, generator=g) * 2.5 / (0.2 * cin * k * k) ** 0.5).to(dtype)
@@ -92,7 +98,7 @@ def test_an_image_comes_out_the_same_wherever_it_stands_in_the_batch(form, B, ci
     to a tile or one."""
     from triton_snn_fusion_b200 import _lib as L
     T, cout = 4, 128
-    assert L.conv_kernel_name(T, B, cin, H, W, cout, 3, 1, 1, torch.bfloat16).startswith("conv_split/")
+    assert L.conv_kernel_name(T, B, cin, H, W, cout, 3, 1, 1, torch.bfloat16) == form
     g = torch.Generator().manual_seed(B)
     x = torch.randn(T, 1, H, W, cin, generator=g).bfloat16().expand(T, B, H, W, cin).contiguous().to(DEV)
     w = (torch.randn(cout, 3, 3, cin, generator=g) * 0.06).bfloat16().to(DEV)

@@ -12,6 +12,7 @@
 // The operand layout (128 output channels as M, 8 x 14 pixels of two timesteps as N = 256, taps as shifted descriptors
 // into a 10 x 16 halo tile, two images per tile on maps of at most 7 x 8) is that of the timestep-pair kernel. Which
 // calls come here: conv_split_plan() below.
+#include <atomic>
 #include <type_traits>
 
 #include "conv.cuh"
@@ -516,17 +517,56 @@ int dispatch(const ConvArgs &a, int S, cudaStream_t stream) {
   return v_f32 ? launch<XT, XT, float>(a, S, stream) : launch<XT, XT, XT>(a, S, stream);
 }
 
+// How many clusters of S CTAs run at once, one CTA per SM. A cluster stays inside a GPC, and which SMs a GPC has differs
+// from one GPU to the next, so this is asked of the device: 33 and 15 for S = 4 and 8 on the B200 that the figures below were
+// taken on, not 148 / S. One tile more is a second wave: 128 -> 496 with a shortcut from 128, T = 6, 16 tiles with S = 8
+// took 51 us, the timestep-pair kernel 34. Without a device the figures of that GPU.
+int clusters_at_once(int S) {
+  static std::atomic<int> known[64][3];
+  const int si = S == 2 ? 0 : (S == 4 ? 1 : 2), fallback = S == 2 ? 72 : (S == 4 ? 33 : 15);
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+    (void)cudaGetLastError();
+    return fallback;
+  }
+  int n = known[dev][si].load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(S * 148));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kSmem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)S;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  using BF = __nv_bfloat16;   // every instantiation has the same block and shared memory, one block per SM
+  if (raise_smem_limit_once<conv_split_kernel<BF, BF, BF>>(kSmem) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, conv_split_kernel<BF, BF, BF>, &cfg) != cudaSuccess || n < 1) {
+    (void)cudaGetLastError();
+    n = fallback;
+  }
+  known[dev][si].store(n, std::memory_order_relaxed);
+  return n;
+}
+
 }  // namespace
 
 // Cluster size for a call, 0 where splitting does not pay. Times in microseconds of one launch, measured on B200 and the
-// same for all shapes within 15 %: the timestep-pair kernel takes 6.5 + 0.41 per weight tile and timestep pair of a wave
-// (0.3 and two thirds of the tiles in its two-kernel-rows form for at most 64 channels), odd T on the halo kernel as
-// much per pair of steps. A cluster takes 6.5 + its share of the weight tiles (0.55 each at three or four timesteps at
-// once, 0.41 at one or two) + the exchange, 0.8 + 0.6 per timestep + 0.33 per timestep and row that a CTA owns (this part
-// has nothing to hide behind, which is why two CTAs with seven rows each rarely pay). 512 -> 512 on one 7x7 map, T = 4: 59
-// us against 36 / 23 / 16 with S = 2 / 4 / 8; 256 -> 512 stride 2 on one 14x14 map: 36 against 22 / 16 / 13; 256 -> 256 on
-// nine 8x8 maps, T = 1: 23 against 15 / 11 / 17 (144 CTAs in clusters of eight do not fit at once); 128 -> 128 stride 2 to
-// 7x7, 116 images: 29 against 37 with S = 2. Split only for a clear gain (a tenth).
+// same for all shapes within 15 %. Whole tiles: the timestep-pair kernel takes 6.5 + 0.41 per weight tile and timestep
+// pair of a wave, 4.6 a pair at least (0.3 and two thirds of the tiles in its two-kernel-rows form for at most 64
+// channels), or 17.5 + 11 a pair at least where the LIF divides; odd T on the halo kernel as much per pair of steps; the
+// 1x1 kernel 4.5 + 0.95 per pair (2 more where it divides, and with a residual) + 0.38 per pair and slab. A cluster takes
+// 3.5 (1x1: 3) + per window of up to four steps 3 (2.5) + its share of the weight tiles (0.55 each at three or four
+// timesteps at once, 0.41 at one or two) + the exchange, 0.8 + 0.6 per timestep + 0.33 per timestep and row that a CTA
+// owns (1.05 where the LIF divides, 0.45 for more than three rows at 1x1 in several windows; this part has nothing to
+// hide behind, which is why two CTAs with seven rows each rarely pay). 512 -> 512 on one 7x7 map, T = 4: 59 us against 36
+// / 23 / 16 with S = 2 / 4 / 8; 256 -> 512 stride 2 on one 14x14 map: 36 against 22 / 16 / 13; 256 -> 256 on nine 8x8
+// maps, T = 1: 23 against 15 / 11 / 17 (144 CTAs in clusters of eight do not fit at once); 128 -> 128 stride 2 to 7x7,
+// 116 images: 29 against 37 with S = 2. 1x1: 1408 -> 72 on 14 pixels, T = 12: 59 whole, 28 with S = 8; 640 -> 48 on 120
+// tokens, T = 8: 23 whole, 29 with S = 8 (two windows for ten weight tiles: left whole). Split only for a clear gain (a
+// tenth).
 // A sum over S partial sums rounds elsewhere than the pair kernel's chain, so outputs of a small batch agree with those of
 // a large one to fp32 rounding of the currents, not always bit for bit. Within a batch an image's place does not matter.
 int conv_split_plan(const ConvArgs &a) {
@@ -535,20 +575,33 @@ int conv_split_plan(const ConvArgs &a) {
   const double tiles = (stack ? (a.B + 1) / 2 : (double)a.B * ((a.Ho + kRows - 1) / kRows) * ((a.Wo + 7) / 8)) * ((a.Cout + 127) / 128);
   const int sms = sm_count() > 0 ? sm_count() : 148;
   if (tiles > sms / 2) return 0;
-  const int ntaps = a.KH * a.KW, kslabs = (a.Cin + 63) / 64;
+  const int ntaps = a.KH * a.KW, kslabs = (a.Cin + 63) / 64, pairs = (a.T + 1) / 2;
   const int nws = kslabs * ntaps + (a.sc_x != nullptr ? a.sc_cin / 64 : 0);
   const bool twin = a.Cout <= 64 && ntaps == 9 && a.stride == 1 && a.sc_x == nullptr;
-  const double pair = (twin ? 6 * kslabs * 0.3 : nws * 0.41) * ((a.T + 1) / 2);   // one wave
-  const int tw = a.T < kMaxTw ? a.T : kMaxTw, nwin = (a.T + tw - 1) / tw;
+  const bool divides = a.lif && a.p.mode == 2;   // tau no power of two: the epilogue is the longer part of a pair
+  const double pair = twin ? 6 * kslabs * 0.3 : (nws > 11 ? nws * 0.41 : 4.6);
+  double whole = 6.5 + pairs * pair;                                                           // conv_pair_impl.cuh
+  if (divides) whole = 17.5 + pairs * (pair > 11 ? pair : 11.0);
+  if (ntaps == 1)                                                                              // conv_pw.cu, one wave
+    whole = 4.5 + pairs * (0.95 + 0.38 * kslabs + (divides ? 2.0 : 0.0) + (a.res != nullptr ? 2.0 : 0.0));
+  const int nwin = (a.T + kMaxTw - 1) / kMaxTw;
   const int rows = (a.Ho < kRows ? a.Ho : kRows) * (stack && a.B > 1 ? 2 : 1);
+  // odd T, where the channel counts rule out the halo and the general kernel too: the CUDA cores take twenty times as long
+  const char *why = "";
+  const bool alone = ntaps == 9 && a.T % 2 != 0 && a.T != 1 && !conv3x3_halo_supported(a) && !conv_lif_tc_supported(a, &why);
   int best = 0;
-  double best_us = 0.9 * (6.5 + pair);
+  double best_us = alone ? 1e300 : 0.9 * whole;
   for (int S = 2; S <= 8 && S <= nws; S *= 2) {
-    const double fit = S == 8 ? 16 : (sms - 4) / S;   // clusters that run at once (a cluster stays inside a GPC)
-    if (tiles > fit) break;
-    const double us = 6.5 + nwin * ((nws + S - 1) / S * (tw > 2 ? 0.55 : 0.41) + 0.8 + 0.6 * tw + 0.33 * tw * ((rows + S - 1) / S));
-    if (us < best_us) {
-      best_us = us;
+    const int at_once = clusters_at_once(S), waves = ((int)tiles + at_once - 1) / at_once;
+    const int share = (nws + S - 1) / S, owned = (rows + S - 1) / S;
+    const double row_us = divides ? 1.05 : (ntaps == 1 && nwin > 1 && owned > 3 ? 0.45 : 0.33);
+    double us = (ntaps == 1 ? 3.0 : 3.5) + (ntaps == 1 ? 2.5 : 3.0) * nwin;
+    for (int win = 0; win < nwin; ++win) {
+      const int tw = a.T - win * kMaxTw < kMaxTw ? a.T - win * kMaxTw : kMaxTw;
+      us += share * (tw > 2 ? 0.55 : 0.41) + 0.8 + tw * (0.6 + row_us * owned);
+    }
+    if (us * waves < best_us) {
+      best_us = us * waves;
       best = S;
     }
   }
