@@ -381,8 +381,8 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
   const bool dup = DUP || (S2 && g.dup);
   // The nine-tap loops of the weight producer and the MMA issuer stay loops: unrolled they compete with the epilogue for
   // the instruction cache (64 -> 128, 16x16, batch 415: 106 us as a loop, 123 us unrolled; the six groups of the twin form:
-  // 123 us as a loop, 117 us unrolled).
-  constexpr int kTapUnroll = TWIN ? 6 : (S2 ? 4 : 1);
+  // 123 us as a loop, 117 us unrolled; stride 2, 128 -> 488, 36x36, batch 7, T = 8: 88 us as a loop, 99 us unrolled by four).
+  constexpr int kTapUnroll = TWIN ? 6 : 1;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bars[2 * kPairRing + 2 * kWBarsP + 4];
   __shared__ uint32_t tmem_base_s;
