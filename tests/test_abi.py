@@ -55,7 +55,7 @@ def test_kernel_choice_is_reported_without_a_gpu():
 
 
 def test_kernel_choice_of_calls_with_few_tiles_and_of_1x1_convs():
-    """The lines that the dispatch draws between the split kernel and those that compute whole tiles, with the
+    """The lines that the dispatch draws between the split, the 1x1 and the general kernel, with the
     cluster counts of the B200 that they were measured on (15 and 33 clusters of 8 and 4 at a time)."""
     import pytest
     import torch
@@ -70,3 +70,7 @@ def test_kernel_choice_of_calls_with_few_tiles_and_of_1x1_convs():
     assert name(3, 8, 192, 9, 9, 24, 3, 1, 1, bf).startswith("conv_split/")  # odd T, 24 channels: nothing else takes it
     assert name(8, 1, 640, 15, 8, 48, 1, 1, 0, bf) == "conv_pw"              # two windows for ten weight tiles do not pay
     assert name(12, 14, 1408, 1, 1, 72, 1, 1, 0, bf) == "conv_split/8"
+    assert name(12, 3, 64, 4, 4, 256, 1, 1, 0, bf) == "conv_lif_tc"          # one slab, six pairs, few tiles
+    assert name(4, 3, 64, 4, 4, 256, 1, 1, 0, bf) == "conv_pw"
+    assert name(4, 9, 64, 4, 4, 16, 1, 1, 0, bf) == "conv_lif_tc"            # sixteen channels out
+    assert name(12, 3, 72, 4, 4, 256, 1, 1, 0, bf) == "conv_pw"              # (the general kernel needs Cin % 64 = 0)

@@ -73,8 +73,9 @@ bool conv3x3_pair_supported(const ConvArgs &a);
 bool pair_shape_supported(const ConvArgs &a);   // the shapes of its tiles, any T; 1x1 too, for conv_split.cu
 int conv3x3_pair(const ConvArgs &a, cudaStream_t stream);
 int pair_device_status(int *out);
-// The form of it for 1x1 convs and linear layers, any T (conv_pw.cu).
+// The form of it for 1x1 convs and linear layers, any T (conv_pw.cu), and where the general kernel is faster.
 bool conv_pw_supported(const ConvArgs &a);
+bool conv_tc_beats_pw(const ConvArgs &a);
 int conv_pw(const ConvArgs &a, cudaStream_t stream);
 int pw_device_status(int *out);
 // The form of it for calls with few output tiles (conv_split.cu): the reduction of a tile over a cluster of CTAs.

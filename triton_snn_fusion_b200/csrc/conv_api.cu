@@ -24,7 +24,7 @@ Kernel choose(const ConvArgs &a, int path, int *S, const char **why) {
   if (path == SNNB_PATH_SIMT) return cuda_cores;
   if (path != SNNB_PATH_TCGEN05_TAPS && path != SNNB_PATH_TCGEN05_HALO) {
     if ((*S = conv_split_plan(a)) != 0) return Kernel::split;
-    if (conv_pw_supported(a)) return Kernel::pw;
+    if (conv_pw_supported(a) && !(conv_lif_tc_supported(a, why) && conv_tc_beats_pw(a))) return Kernel::pw;
     if (conv3x3_pair_supported(a)) return Kernel::pair;
   }
   if (path != SNNB_PATH_TCGEN05_TAPS && conv3x3_halo_supported(a)) return Kernel::halo;

@@ -564,6 +564,17 @@ bool conv_pw_supported(const ConvArgs &a) {
   return aligned16(a.x) && aligned16(a.w);
 }
 
+// Calls that the general kernel of conv_tc.cu, which takes all timesteps of a tile at once and stores 32 bytes of a pixel at
+// a time, does better (measured on B200 over drawn calls, geometric means): at most 16 channels out use 16 of the 128 rows
+// here and a warp's stores fill half a sector pair (Cin 64: its time 0.82 of this kernel's, Cin 128: 0.95, Cin 192: 1.1);
+// with one slab and T >= 9 a tile that has an SM to itself is a chain of five or more epilogues (0.68 with at most a quarter
+// as many tiles as SMs, 1.4 with more; T 7, 8: 0.95; T 5, 6: 1.05).
+bool conv_tc_beats_pw(const ConvArgs &a) {
+  const int sms = sm_count() > 0 ? sm_count() : 148;
+  const long long tiles = ((long long)a.B * a.H * a.W + 127) / 128 * ((a.Cout + 127) / 128);
+  return (tiles <= sms && a.Cout <= 16 && a.Cin <= 128) || (tiles <= sms / 4 && a.Cin <= 64 && a.T >= 9);
+}
+
 int conv_pw(const ConvArgs &a, cudaStream_t stream) {
   return a.dtype == SNNB_BF16 ? dispatch<__nv_bfloat16>(a, stream) : dispatch<__half>(a, stream);
 }
