@@ -55,14 +55,14 @@ def test_kernel_choice_is_reported_without_a_gpu():
 
 
 def test_kernel_choice_of_calls_with_few_tiles_and_of_1x1_convs():
-    """The lines that the dispatch draws between the split, the 1x1 and the general kernel, with the
+    """The lines that the dispatch draws between the split, the 1x1, the general and the two fp32 kernels, with the
     cluster counts of the B200 that they were measured on (15 and 33 clusters of 8 and 4 at a time)."""
     import pytest
     import torch
     from triton_snn_fusion_b200 import _lib
     if torch.cuda.is_available():
         pytest.skip("the cluster counts are those of the GPU at hand")
-    bf, name = torch.bfloat16, _lib.conv_kernel_name
+    bf, f32, name = torch.bfloat16, torch.float32, _lib.conv_kernel_name
     assert name(4, 1, 512, 7, 7, 512, 3, 1, 1, bf) == "conv_split/8"
     assert name(6, 2, 128, 11, 11, 488, 3, 1, 1, bf) != "conv_split/8"       # 16 tiles: one cluster of eight too many
     assert name(4, 8, 512, 7, 7, 512, 3, 1, 1, bf) == "conv_split/4"
@@ -74,3 +74,7 @@ def test_kernel_choice_of_calls_with_few_tiles_and_of_1x1_convs():
     assert name(4, 3, 64, 4, 4, 256, 1, 1, 0, bf) == "conv_pw"
     assert name(4, 9, 64, 4, 4, 16, 1, 1, 0, bf) == "conv_lif_tc"            # sixteen channels out
     assert name(12, 3, 72, 4, 4, 256, 1, 1, 0, bf) == "conv_pw"              # (the general kernel needs Cin % 64 = 0)
+    assert name(5, 24, 8, 39, 39, 336, 1, 1, 0, f32) == "conv_lif_simt"      # K = 8: stores
+    assert name(5, 24, 36, 39, 39, 336, 1, 1, 0, f32).startswith("conv_lif_f32/")
+    assert name(4, 1, 16, 16, 16, 126, 1, 1, 0, f32, one_frame=True) == "conv_lif_simt"
+    assert name(4, 1, 68, 16, 16, 126, 1, 1, 0, f32, one_frame=True).startswith("conv_lif_f32/")

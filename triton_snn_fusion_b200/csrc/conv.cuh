@@ -46,9 +46,10 @@ inline int channel_tile(int most, int Tacc) {
 // CUDA-core implicit GEMM (any shape, fp32 accumulate).
 int conv_lif_simt(const ConvArgs &a, cudaStream_t stream);
 
-// The fp32 form of it with asynchronous copies and packed multiply-adds.
+// The fp32 form of it with asynchronous copies and packed multiply-adds, and where it is the faster one of the two.
 struct F32Tile { int TT, TN; };   // steps of a window, eighths of the channels of a block
 bool conv_f32_supported(const ConvArgs &a);
+bool conv_f32_pays(const ConvArgs &a);
 F32Tile conv_f32_tile(const ConvArgs &a);
 int conv_f32(const ConvArgs &a, cudaStream_t stream);
 

@@ -19,7 +19,7 @@ enum class Kernel { smallcin, simt, f32, split, pw, pair, halo, taps, none };
 
 // The kernel of a call. `S`: cluster size of the split kernel; `why`: what keeps a call with none off the tensor cores.
 Kernel choose(const ConvArgs &a, int path, int *S, const char **why) {
-  const Kernel cuda_cores = conv_f32_supported(a) ? Kernel::f32 : Kernel::simt;
+  const Kernel cuda_cores = conv_f32_supported(a) && conv_f32_pays(a) ? Kernel::f32 : Kernel::simt;
   if (path == SNNB_PATH_AUTO && conv_smallcin_supported(a)) return Kernel::smallcin;   // RGB first layers
   if (path == SNNB_PATH_SIMT) return cuda_cores;
   if (path != SNNB_PATH_TCGEN05_TAPS && path != SNNB_PATH_TCGEN05_HALO) {

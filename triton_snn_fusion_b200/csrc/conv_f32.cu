@@ -23,7 +23,8 @@
 // their own fixed latencies (two warps per scheduler at 255 registers; four at 128 registers gain nothing, because the
 // smaller tile reads more shared memory per multiply-add).
 //
-// Calls with Cin % 4 != 0 or operands off the 16-byte grid stay on the kernel of conv_simt.cu.
+// Calls with Cin % 4 != 0 or operands off the 16-byte grid stay on the kernel of conv_simt.cu, and so do those that are mostly
+// stores (conv_f32_pays).
 #include "conv.cuh"
 
 namespace snnb {
@@ -296,6 +297,21 @@ bool conv_f32_supported(const ConvArgs &a) {
   return a.dtype == SNNB_F32 && a.Cin % 4 == 0 && a.x_t_stride % 4 == 0 && aligned16(a.x) && aligned16(a.w) &&
          a.pad < a.KH && a.pad < a.KW && a.KH <= 128 && a.KW <= 128 && a.H < 16384 && a.W < 16384 && a.stride * (long long)a.Ho < 32768 && a.stride * (long long)a.Wo < 32768 &&
          (128 / ((long long)a.Ho * a.Wo) + 2) * a.H * a.W * a.Cin < (1LL << 31) && !a.xs_w && !a.xs_h && !a.xs_b && !a.xd_w && !a.xd_h && a.sc_x == nullptr;
+}
+
+// Where the kernel of conv_simt.cu is the faster one: with a short K a call is its stores, which that kernel's small blocks
+// (64 pixels, eight to an SM) keep going while these have two to four blocks of 128 rows. Measured on B200, its time against
+// this one's: 8 -> 336 channels, 36504 pixels, T = 5 209 and 346 us; 8 -> 1106, 1452 tokens, T = 2 18 and 34 us; 16 -> 192, 4116
+// pixels, T = 6 29 and 35 us; with few channels out or K = 28 .. 64 about as often one as the other (16 -> 4, 87025 pixels
+// 88 and 49 us; 32 -> 328, 2009 pixels 49 and 41 us). One frame for all steps, where T frames are stored per convolution:
+// K = 16, 126 channels, 6720 pixels, T = 4 17 and 35 us; K = 80, 312 channels, 8325 pixels, T = 6 66 and 107 us; K = 64,
+// 48 channels, 8112 pixels, T = 4 21 and 18 us; 24 -> 37, 14 pixels, T = 12 36 and 9 us.
+bool conv_f32_pays(const ConvArgs &a) {
+  const long long K = (long long)a.KH * a.KW * a.Cin;
+  const long long pixels = (long long)a.B * a.Ho * a.Wo;
+  if (a.x_t_stride == 0 && a.T > 1) return K > 16 * a.T || pixels < 128;
+  const long long blocks = (pixels + 63) / 64 * ((a.Cout + 63) / 64);   // of conv_simt.cu
+  return !(K <= 24 && a.Cout > 96 && blocks >= (sm_count() > 0 ? sm_count() : 148));
 }
 
 namespace {
