@@ -99,25 +99,28 @@ def test_avgpool_linear_mean_arbitrary_values(N):
 
 
 @pytest.mark.gpu
-def test_bounded_wait_runs_out_and_reports():
-    """A wait inside the tcgen05 conv kernel that can never complete (a weight tile that is announced but not
+@pytest.mark.parametrize("kernel,B,cin,k,H", [("conv3x3_pair", 40, 64, 3, 16), ("conv_split/8", 2, 256, 3, 8), ("conv_pw", 2, 128, 1, 16)])
+def test_bounded_wait_runs_out_and_reports(kernel, B, cin, k, H):
+    """A wait inside each of the tcgen05 conv kernels that can never complete (an operand tile that is announced but not
     loaded, limit shortened to about a millisecond) must end by itself: the call returns, the status word says
-    that a wait gave up, and the next call works and leaves the status clean."""
+    that a wait gave up, and the next call works and leaves the status clean. In the split kernel one CTA of a cluster
+    gives up while the others go on to the cluster barriers."""
     from oracle import snn_oracle as orc
     from triton_snn_fusion_b200 import _lib as L
     from util import check_parity
     dtype = torch.bfloat16
     g = torch.Generator().manual_seed(1)
-    x = (torch.rand(4, 2, 16, 16, 64, generator=g) < 0.2).to(dtype)
-    w = (torch.randn(128, 3, 3, 64, generator=g) * 0.12).to(dtype)
+    x = (torch.rand(4, B, H, H, cin, generator=g) < 0.2).to(dtype)
+    w = (torch.randn(128, k, k, cin, generator=g) * 2.88 / (cin * k * k) ** 0.5).to(dtype)
     b = (torch.randn(128, generator=g) * 0.1).to(dtype)
     xd, wd, bd = x.cuda(), w.cuda(), b.cuda()
-    spikes = torch.zeros(4, 2, 16, 16, 128, dtype=dtype, device="cuda")
-    v = torch.zeros(2, 16, 16, 128, dtype=dtype, device="cuda")
+    spikes = torch.zeros(4, B, H, H, 128, dtype=dtype, device="cuda")
+    v = torch.zeros(B, H, H, 128, dtype=dtype, device="cuda")
+    assert L.conv_kernel_name(4, B, cin, H, H, 128, k, 1, k // 2, dtype) == kernel
 
     def call():
         L.check(L.lib.snnb_conv_lif(xd.data_ptr(), xd.stride(0), wd.data_ptr(), bd.data_ptr(), None, None,
-                                    spikes.data_ptr(), v.data_ptr(), 4, 2, 64, 16, 16, 128, 3, 3, 1, 1, 1,
+                                    spikes.data_ptr(), v.data_ptr(), 4, B, cin, H, H, 128, k, k, 1, k // 2, 1,
                                     L.BF16, L.BF16, L.BF16, 1.0, 0.0, 2.0, L.PATH_TCGEN05, None), "snnb_conv_lif")
         torch.cuda.synchronize()
 
@@ -131,7 +134,7 @@ def test_bounded_wait_runs_out_and_reports():
     call()                               # the hook disarmed itself: a normal run
     assert L.device_status() == 0
     rs, rv = orc.temporal_conv_lif([orc.widen(x[t]).permute(0, 3, 1, 2) for t in range(4)],
-                                   orc.widen(w).permute(0, 3, 1, 2), orc.widen(b), None, [1, 1], [1, 1], [1, 1], 1,
+                                   orc.widen(w).permute(0, 3, 1, 2), orc.widen(b), None, [1, 1], [k // 2] * 2, [1, 1], 1,
                                    1.0, 0.0, 2.0)
     check_parity(spikes.permute(0, 1, 4, 2, 3), v.permute(0, 3, 1, 2), rs, rv, dtype, what="after the self-test")
 

@@ -15,9 +15,9 @@ DEV = "cuda"
 
 @pytest.fixture(autouse=True, params=["tcgen05", "tcgen05_halo", "tcgen05_taps"])
 def _force_tc_path(request):
-    """Every case runs with the preferred tensor-core kernel for its shape (3x3/s1 convs with T in {1,2,4}
-    take the timestep-pair kernel), with the halo kernel forced where it applies, and with the general
-    one-load-per-tap kernel forced."""
+    """Every case runs with the preferred tensor-core kernel for its shape (with the few output tiles that most cases here
+    have, the split kernel; test_pair_kernel_at_larger_batches is the timestep-pair kernel's), with the halo kernel
+    forced where it applies, and with the general one-load-per-tap kernel forced."""
     from triton_snn_fusion_b200 import _lib
     from triton_snn_fusion_b200.runtime import triton_convlif_backend as be
     prev = be.set_conv_path(request.param)
@@ -75,14 +75,14 @@ CONV = [
     (2, 128, 256, 3, 2, 1, 28, 28),
     (3, 256, 256, 3, 1, 1, 14, 14),
     (3, 256, 512, 3, 2, 1, 14, 14),
-    (5, 512, 512, 3, 1, 1, 7, 7),        # two images per tile in the pair kernel, odd batch
+    (5, 512, 512, 3, 1, 1, 7, 7),        # two images per tile, odd batch
     (4, 128, 192, 3, 1, 1, 7, 8),        # same, full-width map, partial channel tile
     (3, 64, 128, 3, 1, 1, 4, 6),         # same, small map
     (2, 64, 128, 1, 1, 0, 28, 28),
     (2, 128, 64, 1, 1, 0, 13, 17),
     (1, 64, 48, 3, 1, 1, 9, 11),
     (2, 64, 64, 3, 2, 1, 15, 13),
-    (2, 64, 128, 3, 2, 1, 17, 19),       # stride 2 on odd sizes through the phase views of the pair kernel
+    (2, 64, 128, 3, 2, 1, 17, 19),       # stride 2 on odd sizes through phase views
     (3, 128, 192, 3, 2, 1, 12, 16),      # stride 2 down to a 6x8 map: two images per tile
     (1, 64, 32, 5, 1, 2, 12, 12),
 ]
@@ -314,11 +314,11 @@ def test_membrane_updated_in_place_on_shifted_tiles():
 
 @pytest.mark.parametrize("case", [(2, 32, 64, 28, 28), (2, 96, 128, 16, 16), (3, 40, 192, 14, 14)])
 def test_pointwise_conv_with_a_partial_channel_slab(case):
-    """1x1 convs whose input channels are not a multiple of 64 (MobileNet's first pointwise layer reads 32): the
-    timestep-pair kernel completes the last 64-channel slab of both operands with zeros."""
+    """1x1 convs whose input channels are not a multiple of 64 (MobileNet's first pointwise layer reads 32): the last
+    64-channel slab of both operands is completed with zeros."""
     be = _conv_be()
     if be._conv_path != "tcgen05":
-        pytest.skip("only the timestep-pair kernel takes partial slabs")
+        pytest.skip("only the 1x1 kernel takes partial slabs")
     B, cin, cout, H, W = case
     T, dtype = 4, torch.bfloat16
     torch.manual_seed(cin + cout)
@@ -393,3 +393,63 @@ def test_channel_tiles_that_are_halved_for_many_timesteps(case):
     torch.cuda.synchronize()
     check_parity(sp.permute(0, 1, 4, 2, 3), v.permute(0, 3, 1, 2), rs, rv, dtype, what=str(case))
     assert 0.02 < float(rs.mean()) < 0.6
+
+
+PAIR = [
+    # T, B, cin, cout, stride, H, W, residual ("conv": a 1x1 shortcut conv of stride 2 over 128 channels): batches with so
+    # many tiles that the split kernel leaves them to the timestep-pair kernel
+    (4, 20, 64, 128, 1, 28, 28, True),      # identity residual, strips and row tiles that overlap
+    (4, 24, 256, 256, 1, 14, 14, True),     # four slabs, two channel tiles
+    (4, 81, 64, 192, 1, 7, 7, False),       # two images per tile, odd batch, partial channel tile
+    (2, 81, 64, 192, 1, 7, 8, True),        # the same with a residual, one pair
+    (4, 79, 128, 192, 2, 12, 16, False),    # stride 2 to 6x8: two images per tile
+    (4, 80, 64, 128, 2, 17, 19, True),      # stride 2 on odd sizes
+    (4, 81, 128, 192, 1, 7, 7, "conv"),     # fused shortcut, two images per tile
+    (2, 40, 64, 256, 1, 9, 13, "conv"),     # fused shortcut, one image
+    (1, 40, 64, 130, 1, 14, 14, "conv"),
+    (1, 40, 64, 128, 1, 14, 14, False), (2, 40, 64, 128, 1, 14, 14, False), (6, 40, 64, 128, 1, 14, 14, True),
+    (12, 40, 64, 128, 1, 14, 14, False),    # six pairs
+]
+
+
+@pytest.mark.parametrize("case", PAIR)
+def test_pair_kernel_at_larger_batches(case):
+    from triton_snn_fusion_b200 import _lib as L
+    be = _conv_be()
+    if be._conv_path != "tcgen05":
+        pytest.skip("the other paths have their cases above")
+    T, B, cin, cout, s, H, W, residual = case
+    dtype = torch.bfloat16
+    shortcut = residual == "conv"
+    assert L.conv_kernel_name(T, B, cin, H, W, cout, 3, s, 1, dtype, residual=residual is True) == "conv3x3_pair"
+    g = torch.Generator().manual_seed(B + cin + cout + H)
+    nhwc = lambda t: t.transpose(-3, -2).transpose(-2, -1).contiguous().to(DEV)
+    ho, wo = (H - 1) // s + 1, (W - 1) // s + 1
+    x = (torch.rand(T, B, cin, H, W, generator=g) < 0.15).to(dtype)
+    w = (torch.randn(cout, cin, 3, 3, generator=g) * (2.0 / (cin * 9)) ** 0.5 * 2.5).to(dtype)
+    b = (torch.randn(cout, generator=g) * 0.1).to(dtype)
+    v0 = (torch.randn(B, cout, ho, wo, generator=g) * 0.3).to(dtype)
+    res = (torch.rand(T, B, cout, ho, wo, generator=g) < 0.2).to(dtype) if residual is True else None
+    added = [orc.widen(r) for r in res] if res is not None else None
+    if shortcut:
+        sx = (torch.rand(T, B, 128, 2 * H, 2 * W, generator=g) < 0.15).to(dtype)
+        sw = (torch.randn(cout, 128, 1, 1, generator=g) * 0.2).to(dtype)
+        sb = (torch.randn(cout, generator=g) * 0.1).to(dtype)
+        added = list(orc.temporal_conv_only([orc.widen(f) for f in sx], orc.widen(sw), orc.widen(sb), [2, 2], [0, 0]))
+    rs, rv = orc.temporal_conv_lif([orc.widen(f) for f in x], orc.widen(w), orc.widen(b), orc.widen(v0), [s, s], [1, 1], [1, 1], 1,
+                                   1.0, 0.0, 2.0, residuals=added)
+    xd, wd, bd, vd = nhwc(x), nhwc(w), b.to(DEV), nhwc(v0)
+    sp, v = torch.empty(T, B, ho, wo, cout, dtype=dtype, device=DEV), torch.empty_like(vd)
+    if shortcut:
+        sxd, swd, sbd = nhwc(sx), nhwc(sw), sb.to(DEV)
+        L.check(L.lib.snnb_conv3x3_shortcut_lif(xd.data_ptr(), xd.stride(0), wd.data_ptr(), bd.data_ptr(), sxd.data_ptr(), sxd.stride(0),
+                                                swd.data_ptr(), sbd.data_ptr(), 128, 2 * H, 2 * W, 2, vd.data_ptr(), sp.data_ptr(),
+                                                v.data_ptr(), T, B, cin, H, W, cout, L.BF16, L.BF16, L.BF16, 1.0, 0.0, 2.0, None), "shortcut")
+    else:
+        rd = nhwc(res) if res is not None else None
+        L.check(L.lib.snnb_conv_lif(xd.data_ptr(), xd.stride(0), wd.data_ptr(), bd.data_ptr(), L.ptr(rd), vd.data_ptr(), sp.data_ptr(),
+                                    v.data_ptr(), T, B, cin, H, W, cout, 3, 3, s, 1, 1, L.BF16, L.BF16, L.BF16, 1.0, 0.0, 2.0,
+                                    L.PATH_TCGEN05, None), "conv")
+    torch.cuda.synchronize()
+    check_parity(sp.permute(0, 1, 4, 2, 3), v.permute(0, 3, 1, 2), rs, rv, dtype, what=str(case))
+    assert 0.01 < float(rs.mean()) < 0.7
