@@ -30,7 +30,7 @@ SNNB_PAIR_UNITS(SNNB_PAIR_DECL)
 bool pair_shape_supported(const ConvArgs &a) {
   if (a.dtype != SNNB_BF16 && a.dtype != SNNB_F16) return false;
   const bool k3 = a.KH == 3 && a.KW == 3 && a.stride == 1 && a.pad == 1;
-  const bool k1 = a.KH == 1 && a.KW == 1 && a.stride == 1 && a.pad == 0;   // (conv_split.cu only)
+  const bool k1 = a.KH == 1 && a.KW == 1 && a.stride == 1 && a.pad == 0;   // for conv_split.cu only
   // stride 2: four phase views of the input per slab; the base of the odd-column views must stay 16-byte aligned
   const bool k3s2 = a.KH == 3 && a.KW == 3 && a.stride == 2 && a.pad == 1 && a.Cout > 64 && a.H >= 2 && a.W >= 2;
   if (!k3 && !k1 && !k3s2) return false;

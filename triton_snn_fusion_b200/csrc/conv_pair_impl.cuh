@@ -1,8 +1,8 @@
 // 3x3 / padding 1 conv, stride 1 or 2 (+ bias, + residual) + LIF over T steps (T = 1 or even) with the operand roles
 // swapped so that one tcgen05.mma covers 256 output pixels.
 //
-// Measured on B200: a tcgen05.mma (cta_group::1, K = 16) occupies the tensor pipe for ~128 cycles
-// whether its N is 64, 128 or 256, so only N = 256 instructions reach the pipe's rate. With output
+// Measured on B200: a tcgen05.mma (cta_group::1, M = 128, K = 16) with N = 256 occupies the tensor pipe for 128 cycles, one
+// with N = 128 and a fresh operand tile for 113, so only N = 256 comes near the pipe's rate. With output
 // pixels as the M dimension (conv_tc.cu, conv_halo.cu) N is the channel tile and T accumulators of
 // 256 columns do not fit the 512 TMEM columns. Here the weight tile is the M operand (128 output
 // channels, rows beyond Cout are zero) and the pixels of TWO consecutive timesteps are the N operand:
@@ -86,8 +86,8 @@ struct PairGeom {
               // of D1 / D2 for 32 channels; the warps of quarters q and q ^ 1 pass each other through shared memory
               // the halves the other one needs and each runs the LIF for a quarter of the tile's rows.
   int stage_off;   // twin: byte offset of the exchange buffers from the aligned start of dynamic shared memory
-  int dup;    // Cout <= 64 (shapes twin mode does not take): the 64 weight rows are loaded twice (M rows 64..127 repeat 0..63) so that all
-              // eight epilogue warps can read the accumulator and split the pixels four ways
+  int dup;    // Cout <= 64 with the twin mode switched off: the 64 weight rows are loaded twice (M rows 64..127 repeat 0..63) so
+              // that all eight epilogue warps can read the accumulator and split the pixels four ways
   long long wait_limit;   // bound of every mbarrier wait, in SM cycles (about two seconds unless a self-test shortens it)
   int drop_load;          // self-test: CTA 0 announces its first weight tile but never loads it, so that its waits run out
   int own;    // v_init and v_out are the same buffer: a tile that was shifted back inside the image leaves the
@@ -367,8 +367,9 @@ __device__ __forceinline__ void twin_step(const LifParams &p, uint32_t tmem_addr
   }
 }
 
-// DUP: the instantiation for duplicated weight rows at stride 1 (a thread owns four tile rows, 32 membrane values);
-// strided convs with at most 64 outputs run the S2 instantiation, which handles that case at run time.
+// DUP: the instantiation with duplicated weight rows (a thread owns four tile rows, 32 membrane values). It exists for
+// comparison: SNNB_TWIN=0 in the environment selects it for the 3x3 / stride 1 convs with at most 64 outputs that run the
+// twin form otherwise, and no other call has so few outputs here.
 template <typename XT, typename ST, typename VT, bool S2, bool TWIN, bool DUP>
 __global__ void __launch_bounds__(Roles<TWIN>::kThreads)
 conv3x3_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
@@ -378,7 +379,7 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
                     const XT *__restrict__ bias, const XT *__restrict__ bias2, const VT *v_init,
                     ST *__restrict__ spikes, VT *v_out, const PairGeom g, const LifParams p) {
   using R = Roles<TWIN>;
-  const bool dup = DUP || (S2 && g.dup);
+  constexpr bool dup = DUP;
   // The nine-tap loops of the weight producer and the MMA issuer stay loops: unrolled they compete with the epilogue for
   // the instruction cache (64 -> 128, 16x16, batch 415: 106 us as a loop, 123 us unrolled; the six groups of the twin form:
   // 123 us as a loop, 117 us unrolled; stride 2, 128 -> 488, 36x36, batch 7, T = 8: 88 us as a loop, 99 us unrolled by four).
@@ -839,8 +840,7 @@ conv3x3_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
             done = true;
           }
         }
-        if constexpr (DUP) {   // duplicated weight rows at stride 1: four or two tile rows per thread (strided convs
-                               // with at most 64 outputs take the general body below)
+        if constexpr (DUP) {   // duplicated weight rows: four or two tile rows per thread
           if (!done && lean && g.Cout == 64 && rows_valid <= 4) {
             if (rows_valid == 4) pair_epilogue_lean<ST, 4, 64, NV>(p, taddr, bias_c, out, frame_out, pm, v);
             else pair_epilogue_lean<ST, 2, 64, NV>(p, taddr, bias_c, out, frame_out, pm, v);
