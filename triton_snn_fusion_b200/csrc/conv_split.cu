@@ -556,11 +556,13 @@ int clusters_at_once(int S) {
 // Cluster size for a call, 0 where splitting does not pay. Times in microseconds of one launch, measured on B200 and the
 // same for all shapes within 15 %. Whole tiles: the timestep-pair kernel takes 6.5 + 0.41 per weight tile and timestep
 // pair of a wave, 4.6 a pair at least (0.3 and two thirds of the tiles in its two-kernel-rows form for at most 64
-// channels), or 17.5 + 11 a pair at least where the LIF divides; odd T on the halo kernel as much per pair of steps; the
-// 1x1 kernel 4.5 + 0.95 per pair (2 more where it divides, and with a residual) + 0.38 per pair and slab. A cluster takes
-// 3.5 (1x1: 3) + per window of up to four steps 3 (2.5) + its share of the weight tiles (0.55 each at three or four
-// timesteps at once, 0.41 at one or two) + the exchange, 0.8 + 0.6 per timestep + 0.33 per timestep and row that a CTA
-// owns (1.05 where the LIF divides, 0.45 for more than three rows at 1x1 in several windows; this part has nothing to
+// channels), 17.5 + 11 a pair at least where the LIF divides, 10 + 10 with a soft reset (6.5 a pair in the
+// two-kernel-rows form, whose epilogue has twice the warps); odd T on the halo kernel as much per pair of steps; the 1x1
+// kernel 4.5 + 0.95 per pair (3 more where the LIF divides; 2.0, 0.8 or 0.3 more with a residual whose rows are off
+// 64-byte boundaries, are on them, or have at most 64 channels) + 0.38 per pair and slab. A cluster takes 4.3 (1x1: 3) +
+// per window of up to four steps 2.2 (2.5) + its share of the weight tiles (0.55 each at three or four timesteps at once,
+// 0.41 at one or two) + the exchange, 0.8 + 0.6 per timestep + 0.33 per timestep and row that a CTA owns (1.05 where the
+// LIF divides, 0.6 with a soft reset, 0.45 for more than two rows at 1x1 in several windows; this part has nothing to
 // hide behind, which is why two CTAs with seven rows each rarely pay). 512 -> 512 on one 7x7 map, T = 4: 59 us against 36
 // / 23 / 16 with S = 2 / 4 / 8; 256 -> 512 stride 2 on one 14x14 map: 36 against 22 / 16 / 13; 256 -> 256 on nine 8x8
 // maps, T = 1: 23 against 15 / 11 / 17 (144 CTAs in clusters of eight do not fit at once); 128 -> 128 stride 2 to 7x7,
@@ -578,12 +580,15 @@ int conv_split_plan(const ConvArgs &a) {
   const int ntaps = a.KH * a.KW, kslabs = (a.Cin + 63) / 64, pairs = (a.T + 1) / 2;
   const int nws = kslabs * ntaps + (a.sc_x != nullptr ? a.sc_cin / 64 : 0);
   const bool twin = a.Cout <= 64 && ntaps == 9 && a.stride == 1 && a.sc_x == nullptr;
-  const bool divides = a.lif && a.p.mode == 2;   // tau no power of two: the epilogue is the longer part of a pair
-  const double pair = twin ? 6 * kslabs * 0.3 : (nws > 11 ? nws * 0.41 : 4.6);
-  double whole = 6.5 + pairs * pair;                                                           // conv_pair_impl.cuh
-  if (divides) whole = 17.5 + pairs * (pair > 11 ? pair : 11.0);
-  if (ntaps == 1)                                                                              // conv_pw.cu, one wave
-    whole = 4.5 + pairs * (0.95 + 0.38 * kslabs + (divides ? 2.0 : 0.0) + (a.res != nullptr ? 2.0 : 0.0));
+  // LIF kinds with a longer epilogue: 2 with a division, 1 with a soft reset
+  const int kind = !a.lif ? 0 : (a.p.mode == 2 ? 2 : (a.p.hard ? 0 : 1));
+  const double mma = twin ? 6 * kslabs * 0.3 : nws * 0.41;
+  const double epilogue = twin ? (kind ? 6.5 : 0.0) : (kind == 2 ? 11.0 : (kind == 1 ? 10.0 : 4.6));
+  double whole = (twin || kind == 0 ? 6.5 : (kind == 2 ? 17.5 : 10.0)) + pairs * (mma > epilogue ? mma : epilogue);   // conv_pair_impl.cuh
+  if (ntaps == 1) {                                                                            // conv_pw.cu, one wave
+    const double residual = a.res == nullptr ? 0.0 : (a.Cout <= 64 ? 0.3 : (a.Cout % 32 != 0 ? 2.0 : 0.8));
+    whole = 4.5 + pairs * (0.95 + 0.38 * kslabs + (kind == 2 ? 3.0 : 0.0) + residual);
+  }
   const int nwin = (a.T + kMaxTw - 1) / kMaxTw;
   const int rows = (a.Ho < kRows ? a.Ho : kRows) * (stack && a.B > 1 ? 2 : 1);
   // odd T, where the channel counts rule out the halo and the general kernel too: the CUDA cores take twenty times as long
@@ -594,8 +599,8 @@ int conv_split_plan(const ConvArgs &a) {
   for (int S = 2; S <= 8 && S <= nws; S *= 2) {
     const int at_once = clusters_at_once(S), waves = ((int)tiles + at_once - 1) / at_once;
     const int share = (nws + S - 1) / S, owned = (rows + S - 1) / S;
-    const double row_us = divides ? 1.05 : (ntaps == 1 && nwin > 1 && owned > 3 ? 0.45 : 0.33);
-    double us = (ntaps == 1 ? 3.0 : 3.5) + (ntaps == 1 ? 2.5 : 3.0) * nwin;
+    const double row_us = kind == 2 ? 1.05 : kind == 1 ? 0.6 : (ntaps == 1 && nwin > 1 && owned > 2 ? 0.45 : 0.33);
+    double us = ntaps == 1 ? 3.0 + 2.5 * nwin : 4.3 + 2.2 * nwin;
     for (int win = 0; win < nwin; ++win) {
       const int tw = a.T - win * kMaxTw < kMaxTw ? a.T - win * kMaxTw : kMaxTw;
       us += share * (tw > 2 ? 0.55 : 0.41) + 0.8 + tw * (0.6 + row_us * owned);
