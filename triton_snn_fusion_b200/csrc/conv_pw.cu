@@ -95,8 +95,8 @@ __device__ __forceinline__ void lif16(const uint32_t (&a)[16], const XT (&r)[16]
 // A warp's residuals on their way to it. A thread's own are 2-byte reads from 16 rows, whose latency nothing covers (the
 // registers hold one step's at most), and where the rows do not lie on 64-byte boundaries every one of them touches two or
 // three lines more. There (`on`: Cout % 32 != 0; the copies also need Cout % 8 == 0 and a 16-byte aligned tensor) the
-// steps of 16 pixels x 32 channels (1 KB) are copied to shared memory kResAhead steps before they are used: 112 -> 176
-// channels and the like take 0.75 of the time of direct reads, 64 -> 136, 27900 pixels, T = 4 69 -> 50 us. On 64-byte
+// steps of 16 pixels x 32 channels (1 KB) are copied to shared memory kResAhead steps before they are used: 0.73 of the
+// time of direct reads over drawn calls (64 -> 136, 27900 pixels, T = 4: 68 -> 38 us). On 64-byte
 // boundaries direct reads are the faster ones by 5 to 10 %, and with K > 512 the ring of operands needs the room.
 template <typename XT>
 struct Residuals {
@@ -197,6 +197,7 @@ __device__ __forceinline__ void pair_steps(uint32_t taddr, int tq, int npx, floa
     if (half * 16 < npx) {
 #pragma unroll 1
       for (int q = 0; q < tq; ++q) {
+        __syncwarp();   // predicated work of the step before; the load from tensor memory is the whole warp's
         uint32_t a[16], mk = mask >> (half * 16);
         int pitch = g.Cout;
         asm volatile("" : "+r"(mk), "+r"(pitch));   // what follows from them stays in the loop: 96 registers do not hold it
@@ -316,6 +317,7 @@ __device__ __forceinline__ void epilogue(const PwGeom &g, const LifParams &p, co
         if (mask >> i & 1u) *to = DT<VT>::from_f(v[i]);
     }
   }
+  if (RES && !DIRECT) asm volatile("cp.async.wait_all;" ::: "memory");   // what a wait that gave up left behind
 }
 
 // FORM: the common LIF without a residual, or with one that is read directly, each alone in its kernel; or everything else.
