@@ -86,8 +86,8 @@ int snnb_device_status(int *status_out);
 /*
  * Self-test of those bounded waits (no counterpart in the reference, whose Triton kernels do not wait on
  * barriers of their own). Arms the NEXT snnb_conv_lif / snnb_linear_lif / snnb_conv3x3_shortcut_lif call
- * that runs on the timestep-pair kernel: its waits give up after `limit_cycles` SM cycles (1e3 .. 4e9) instead
- * of about two seconds, and its first thread block announces one weight tile that it never loads. That block's
+ * that runs on the timestep-pair, split or 1x1 kernel: its waits give up after `limit_cycles` SM cycles (1e3 .. 4e9)
+ * instead of about two seconds, and its first thread block announces one operand tile that it never loads. That block's
  * waits therefore run out: it records the fact in the status word, releases its tensor memory and returns,
  * while the other blocks finish normally. Nothing traps, faults or hangs; the armed call returns SNNB_OK, its
  * output is incomplete, and snnb_device_status() then reports a non-zero status once. The call after it runs
@@ -174,9 +174,10 @@ int snnb_dwconv3x3_lif(const void *x_seq, int64_t x_t_stride, const void *w, con
  * `lif` = 0 turns the LIF off: `spikes` then receives conv + bias (+ residual)
  * in the activation dtype for every t and v_init / v_out are ignored (used for
  * the BN-folded shortcut convs that feed a residual input).
- * path: the tensor-core kernels need dtype bf16/f16, Cin % 64 == 0, Cout % 16 == 0,
+ * path: the general tensor-core kernel needs dtype bf16/f16, Cin % 64 == 0, Cout % 16 == 0,
  * stride 1 or 2, kernel at most 11x11 and T accumulators that fit the 512 TMEM
- * columns (T <= 32); anything else runs on SNNB_PATH_SIMT.
+ * columns (T <= 32); 1x1 convs need only Cin % 8 == 0 and 3x3 convs with T = 1 or even (with few
+ * output tiles any T) only Cin % 64 == 0; anything else runs on SNNB_PATH_SIMT.
  */
 int snnb_conv_lif(const void *x_seq, int64_t x_t_stride, const void *w, const void *b,
                   const void *residual, const void *v_init, void *spikes, void *v_out,

@@ -5,7 +5,7 @@ Mirrors the public names of the reference module of the same name
 (runtime/triton_convlif_backend.py in pengjh0111/triton-snn-fusion: result type :7-15,
 classify_conv_lif_config :50-82, check_triton_support :118-211, the run_* entry points
 :331-817), so the reference's op layer binds to it unchanged. Behind the names:
-``snnb_conv_lif`` (tcgen05 implicit GEMM for 16-bit activations with Cin % 64 == 0,
+``snnb_conv_lif`` (tcgen05 kernels for 16-bit activations, mostly with Cin % 64 == 0,
 CUDA-core implicit GEMM otherwise) and ``snnb_dwconv3x3_lif``.
 
 Deliberate differences from the reference backend:
